@@ -13,6 +13,14 @@
 //     warp (lane = row) grows the BFS frontier of the whole tile with shifts,
 //     warp shuffles and ballots, seeded by sink nodes (level 1) and by the
 //     halo's heights.  It gives exact distances for the tile given the halo.
+//   * Height limit: the first outer iterations relabel and push only within a
+//     few steps of the sinks (SolveParams::near_h).  Excess far from any sink
+//     that has capacity left is mostly trapped behind edges that the excess
+//     next to them saturates: moved from the start, it wanders until its
+//     height runs away (on the 256-image batch 85% of the pushes started more
+//     than 16 steps from a sink); left where it is, the termination check
+//     finds it cut off.  What it does not find cut off is moved in a later
+//     iteration, whose limit is four times as high and then none.
 //   * Global relabel (GraphCutKernels.cu:757-875 does 10 Bellman-Ford steps
 //     per launch with a host round trip each): tiles recompute with the tile
 //     BFS until no tile border changes; a tile whose border distances
@@ -198,6 +206,10 @@ struct PhaseClock {
 // hl/hr: level of this row's left/right halo node; ht/hb: level of the halo
 // node above/below column `lane`.
 
+// hlim (in the BFS loops below): no level above it is needed.  A loop stops
+// once its level reaches it; the levels of the last round may lie up to three
+// above it, and every pixel not reached by then gets INF_H.
+
 // One BFS expansion: the nodes outside S that have a residual edge into S or
 // into a halo node of level <= lvl (they get level lvl + 1).
 __device__ __forceinline__ unsigned bfs_expand(unsigned S, int lvl, unsigned Rl, unsigned Rr, unsigned Ru,
@@ -252,7 +264,7 @@ struct GrScratch {
 // tile_bfs_gr); the divergent stores make it the slower one wherever a visit's
 // latency bounds the round.
 __device__ unsigned tile_bfs_direct(unsigned Rl, unsigned Rr, unsigned Ru, unsigned Rd, unsigned sink, int hl,
-                         int hr, int ht, int hb, int *hs, int stride, int *iters) {
+                         int hr, int ht, int hb, int hlim, int *hs, int stride, int *iters) {
     const int lane = threadIdx.x & 31;
     int *row = hs + lane * stride;
     // INF, and level 1 on the seeds, in one uniform pass (a loop over the
@@ -262,7 +274,7 @@ __device__ unsigned tile_bfs_direct(unsigned Rl, unsigned Rr, unsigned Ru, unsig
     unsigned S = sink;
     int lvl = 1;
     int it = 0;
-    for (; it < BFS_MAX_ITERS; ++it) {
+    for (; it < BFS_MAX_ITERS && lvl < hlim; ++it) {
         unsigned nw1 = bfs_expand(S, lvl, Rl, Rr, Ru, Rd, hl, hr, ht, hb, lane);
         const unsigned S1 = S | nw1;
         unsigned nw2 = bfs_expand(S1, lvl + 1, Rl, Rr, Ru, Rd, hl, hr, ht, hb, lane);
@@ -298,8 +310,8 @@ __device__ unsigned tile_bfs_direct(unsigned Rl, unsigned Rr, unsigned Ru, unsig
 // expansions the levels found so far are written out and the planes start a
 // new segment.
 __device__ unsigned tile_bfs_gr(unsigned Rl, unsigned Rr, unsigned Ru, unsigned Rd, unsigned sink, int hl, int hr,
-                                int ht, int hb, int *h, GrScratch &sc, int *iters, int &vt, int &vb, int &vl,
-                                int &vr) {
+                                int ht, int hb, int hlim, int *h, GrScratch &sc, int *iters, int &vt, int &vb,
+                                int &vl, int &vr) {
     const int lane = threadIdx.x & 31;
     unsigned S = sink, base = 0u;
     unsigned P[GR_NPL];
@@ -349,7 +361,7 @@ __device__ unsigned tile_bfs_gr(unsigned Rl, unsigned Rr, unsigned Ru, unsigned 
         base = S;
         nidx = 0;
     };
-    for (; it < BFS_MAX_ITERS; ++it) {
+    for (; it < BFS_MAX_ITERS && lvl < hlim; ++it) {
         const unsigned nw1 = bfs_expand(S, lvl, Rl, Rr, Ru, Rd, hl, hr, ht, hb, lane);
         const unsigned S1 = S | nw1;
         const unsigned nw2 = bfs_expand(S1, lvl + 1, Rl, Rr, Ru, Rd, hl, hr, ht, hb, lane);
@@ -398,14 +410,14 @@ __device__ unsigned tile_bfs_gr(unsigned Rl, unsigned Rr, unsigned Ru, unsigned 
 constexpr int NREC = 64;
 constexpr int NRS = NREC + 1;  // odd row stride: a warp's record stores and searches spread over the banks
 __device__ int tile_bfs_rec(unsigned Rl, unsigned Rr, unsigned Ru, unsigned Rd, unsigned sink, int hl, int hr,
-                            int ht, int hb, int *hs, int stride, unsigned *srec, int *lv, unsigned *sfin,
-                            int *iters) {
+                            int ht, int hb, int hlim, int *hs, int stride, unsigned *srec, int *lv,
+                            unsigned *sfin, int *iters) {
     const int lane = threadIdx.x & 31;
     int *row = hs + lane * stride;
     unsigned *rec = srec + lane * NRS;
     unsigned S = sink;
     int lvl = 1, nrec = 0, it = 0;
-    for (; it < BFS_MAX_ITERS; ++it) {
+    for (; it < BFS_MAX_ITERS && lvl < hlim; ++it) {
         const unsigned nw1 = bfs_expand(S, lvl, Rl, Rr, Ru, Rd, hl, hr, ht, hb, lane);
         const unsigned S1 = S | nw1;
         const unsigned nw2 = bfs_expand(S1, lvl + 1, Rl, Rr, Ru, Rd, hl, hr, ht, hb, lane);
@@ -560,9 +572,10 @@ __device__ __forceinline__ void gr_prefetch(const Batch &b, int t, GrGeo &gg, bo
 // neighbour's facing pixels, through its residual edge into this tile, a
 // shorter path than its current height; the heights read for that are at
 // least current (distances only fall during a relabel), so no needed visit is
-// missed.
-__device__ void gr_run(const Batch &b, int t, const GrGeo &g, bool round0, bool direct, int tag_next, int slot_next,
-                       GrScratch &sc, int *hs, unsigned long long *st) {
+// missed.  Distances above hlim are not passed on, so only heights up to hlim
+// are exact (hlim = INF_H - 1: all of them).
+__device__ void gr_run(const Batch &b, int t, const GrGeo &g, bool round0, bool direct, int hlim, int tag_next,
+                       int slot_next, GrScratch &sc, int *hs, unsigned long long *st) {
     const int lane = threadIdx.x & 31;
     const size_t base = (size_t)t * TPX;
     unsigned m[6];
@@ -592,7 +605,7 @@ __device__ void gr_run(const Batch &b, int t, const GrGeo &g, bool round0, bool 
     int vt, vb, vl, vr;  // the tile's border heights (this lane's column / row)
     unsigned reached;
     if (direct) {  // warp-uniform
-        reached = tile_bfs_direct(m[0], m[1], m[2], m[3], m[4], hl, hr, ht, hb, hs, 33, &its);
+        reached = tile_bfs_direct(m[0], m[1], m[2], m[3], m[4], hl, hr, ht, hb, hlim, hs, 33, &its);
         __syncwarp();
 #pragma unroll 4
         for (int r = 0; r < 32; ++r) b.h[base + r * 32 + lane] = hs[r * 33 + lane];
@@ -601,7 +614,8 @@ __device__ void gr_run(const Batch &b, int t, const GrGeo &g, bool round0, bool 
         vl = hs[lane * 33];
         vr = hs[lane * 33 + 31];
     } else {
-        reached = tile_bfs_gr(m[0], m[1], m[2], m[3], m[4], hl, hr, ht, hb, b.h + base, sc, &its, vt, vb, vl, vr);
+        reached = tile_bfs_gr(m[0], m[1], m[2], m[3], m[4], hl, hr, ht, hb, hlim, b.h + base, sc, &its, vt, vb, vl,
+                              vr);
     }
     if (lane == 0) stat_add(st, ST_BFS_IT_GR, (unsigned long long)its);
     b.hfin[(size_t)t * 32 + lane] = reached;  // finite heights of this row (the extraction's S_max)
@@ -617,10 +631,10 @@ __device__ void gr_run(const Batch &b, int t, const GrGeo &g, bool round0, bool 
         own[HB_RGT + lane] = vr;
     }
     if (!round0) {
-        const bool up_t = __any_sync(FULL, ((fu >> lane) & 1u) && vt < INF_H && vt + 1 < ht);
-        const bool up_b = __any_sync(FULL, ((fd >> lane) & 1u) && vb < INF_H && vb + 1 < hb);
-        const bool up_l = __any_sync(FULL, fl && vl < INF_H && vl + 1 < hl);
-        const bool up_r = __any_sync(FULL, fr && vr < INF_H && vr + 1 < hr);
+        const bool up_t = __any_sync(FULL, ((fu >> lane) & 1u) && vt < hlim && vt + 1 < ht);
+        const bool up_b = __any_sync(FULL, ((fd >> lane) & 1u) && vb < hlim && vb + 1 < hb);
+        const bool up_l = __any_sync(FULL, fl && vl < hlim && vl + 1 < hl);
+        const bool up_r = __any_sync(FULL, fr && vr < hlim && vr + 1 < hr);
         // lanes 0..3 queue the left, right, upper and lower neighbour
         const int nbt = lane == 0 ? g.nb[0] : lane == 1 ? g.nb[1] : lane == 2 ? g.nb[2] : g.nb[3];
         const bool up = lane == 0 ? up_l : lane == 1 ? up_r : lane == 2 ? up_t : up_b;
@@ -638,7 +652,7 @@ __device__ void gr_run(const Batch &b, int t, const GrGeo &g, bool round0, bool 
 // masks), then the image's finished flag and the neighbours' border lines:
 // two memory round trips for the pair where one tile alone took four.  A
 // tile of a finished image is not checked.
-__device__ void gr_pull_check(const Batch &b, int t0, int t1, int tag_next, int slot_next) {
+__device__ void gr_pull_check(const Batch &b, int t0, int t1, int hlim, int tag_next, int slot_next) {
     const int lane = threadIdx.x & 31;
     const int tt[2] = {t0, t1 >= 0 ? t1 : t0};
     int img[2], ot[2], ob[2], ol[2], orr[2];
@@ -667,9 +681,9 @@ __device__ void gr_pull_check(const Batch &b, int t0, int t1, int tag_next, int 
         const int hb = nb[q].w >= 0 ? __ldcg(b.hb + (size_t)nb[q].w * 128 + HB_TOP + lane) : INF_H;
         const int hl = nb[q].x >= 0 ? __ldcg(b.hb + (size_t)nb[q].x * 128 + HB_RGT + lane) : INF_H;
         const int hr = nb[q].y >= 0 ? __ldcg(b.hb + (size_t)nb[q].y * 128 + HB_LFT + lane) : INF_H;
-        const bool imp = (((ru[q] >> lane) & 1u) && ht < INF_H && ht + 1 < ot[q]) ||
-                         (((rd[q] >> lane) & 1u) && hb < INF_H && hb + 1 < ob[q]) ||
-                         (rl[q] && hl < INF_H && hl + 1 < ol[q]) || (rr[q] && hr < INF_H && hr + 1 < orr[q]);
+        const bool imp = (((ru[q] >> lane) & 1u) && ht < hlim && ht + 1 < ot[q]) ||
+                         (((rd[q] >> lane) & 1u) && hb < hlim && hb + 1 < ob[q]) ||
+                         (rl[q] && hl < hlim && hl + 1 < ol[q]) || (rr[q] && hr < hlim && hr + 1 < orr[q]);
         want[q] = !done && __any_sync(FULL, imp);  // done is warp-uniform
     }
     enqueue_warp(b, b.mark_gr, slot_next, tag_next, t0, lane == 0 && want[0]);
@@ -769,7 +783,7 @@ __device__ void sink_reach_tile(const Batch &b, int t, bool round0, int tag_next
 // sweeps end, so that the atomic overlaps the write-back; it is left in s.idx
 // for the caller.
 template <int NW>
-__device__ void push_tile(const Batch &b, int t, const SolveParams &prm, int phase, SmemPush<NW> &s,
+__device__ void push_tile(const Batch &b, int t, const SolveParams &prm, int hlim, int phase, SmemPush<NW> &s,
                           unsigned long long *st, int *take_ctr) {
     constexpr int RPW = TILE_H / NW;  // rows per warp: thread (warp, lane) owns rows warp + NW k, column lane
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -821,8 +835,8 @@ __device__ void push_tile(const Batch &b, int t, const SolveParams &prm, int pha
             int its = 0;
             const int nrec = tile_bfs_rec(s.m[0][lane], s.m[1][lane], s.m[2][lane], s.m[3][lane], s.m[4][lane],
                                           s.h[lane + 1][0], s.h[lane + 1][TILE_W + 1], s.h[0][lane + 1],
-                                          s.h[TILE_H + 1][lane + 1], &s.h[1][1], TILE_W + 2, s.srec, s.lv, s.sfin,
-                                          &its);
+                                          s.h[TILE_H + 1][lane + 1], hlim, &s.h[1][1], TILE_W + 2, s.srec, s.lv,
+                                          s.sfin, &its);
             if (lane == 0) {
                 s.nrec = nrec;
                 stat_add(st, ST_BFS_IT_PUSH, (unsigned long long)its);
@@ -863,7 +877,7 @@ __device__ void push_tile(const Batch &b, int t, const SolveParams &prm, int pha
         for (int k = 0; k < RPW; ++k) {
             const int r = warp + NW * k;
             const int hh = hv[k];
-            if (ev[k] > 0 && hh < INF_H) {
+            if (ev[k] > 0 && hh <= hlim) {
                 const int4 c = s.c[r][lane];
                 const int hl = s.h[r + 1][lane], hr = s.h[r + 1][lane + 2];
                 const int hu = s.h[r][lane + 1], hd = s.h[r + 2][lane + 1];
@@ -932,7 +946,7 @@ __device__ void push_tile(const Batch &b, int t, const SolveParams &prm, int pha
 #pragma unroll
                 for (int k = 0; k < RPW; ++k) {
                     const int r = warp + NW * k;
-                    act |= s.e[r][lane] > 0 && s.h[r + 1][lane + 1] < INF_H;
+                    act |= s.e[r][lane] > 0 && s.h[r + 1][lane + 1] <= hlim;
                 }
                 any = __syncthreads_or(act);
                 if (!any) break;
@@ -952,7 +966,7 @@ __device__ void push_tile(const Batch &b, int t, const SolveParams &prm, int pha
         for (int k = 0; k < RPW; ++k) {
             const int r = warp + NW * k;
             int hh = hv[k];
-            if (ev[k] > 0 && hh < INF_H) {
+            if (ev[k] > 0 && hh <= hlim) {
                 const int4 c = s.c[r][lane];
                 const int hl = s.h[r + 1][lane], hr = s.h[r + 1][lane + 2];
                 const int hu = s.h[r][lane + 1], hd = s.h[r + 2][lane + 1];
@@ -965,7 +979,7 @@ __device__ void push_tile(const Batch &b, int t, const SolveParams &prm, int pha
                     hh = m >= INF_H - 1 ? INF_H : m + 1;
                     s.h[r + 1][lane + 1] = hh;
                 }
-                act |= hh < INF_H;
+                act |= hh <= hlim;
             }
         }
         any = __syncthreads_or(act);
@@ -1198,7 +1212,9 @@ __global__ void __launch_bounds__(NW * 32, solve_min_blocks<NW>()) k_solve(Batch
     int G = 0;  // global relabel round counter (tags of the tile frontier)
     bool finished = false;
     bool timeline = false;  // block 0, thread 0 during the first global relabel: records its timeline
+    bool full = prm.near_outer == 0;  // no height limit any more (grid-uniform)
     for (int outer = 0; outer < prm.max_outer; ++outer) {
+        const int hlim = full || outer >= prm.near_outer ? INF_H - 1 : prm.near_h << (2 * outer);
         if (prm.phase == 2) goto push_rounds;  // the phase-1 launch did the relabel and the count
         if (outer > 0) {
             const int rc = closure_check<NW>(b, prm, G);
@@ -1210,6 +1226,7 @@ __global__ void __launch_bounds__(NW * 32, solve_min_blocks<NW>()) k_solve(Batch
             }
         }
         // ------------------------ exact global relabel ------------------------
+        // (up to hlim: a height above it, or INF, means farther than hlim)
         timeline = prm.phase == 1 && blockIdx.x == 0 && threadIdx.x == 0;  // the phase-split diagnostic
         if (timeline) ctl->gr_time[0] = gtimer();
         for (int k = gtid; k < batch_nimg(b); k += nthreads) {
@@ -1229,7 +1246,8 @@ __global__ void __launch_bounds__(NW * 32, solve_min_blocks<NW>()) k_solve(Batch
             gr_prefetch(b, t, g, true);
             if (g.skip) continue;
             const long long c0 = clock64();
-            gr_run(b, t, g, true, nt >= 2 * nwarps, G + 1, L_GR0 + ((G + 1) & 1), sm.w.g[warp], sm.w.hs[warp], st);
+            gr_run(b, t, g, true, nt >= 2 * nwarps, hlim, G + 1, L_GR0 + ((G + 1) & 1), sm.w.g[warp], sm.w.hs[warp],
+                   st);
             if (lane == 0) {
                 stat_add(st, ST_CYC_GR, (unsigned long long)(clock64() - c0));
                 stat_add(st, ST_GR_TILES, 1ull);
@@ -1240,7 +1258,7 @@ __global__ void __launch_bounds__(NW * 32, solve_min_blocks<NW>()) k_solve(Batch
         for (int k = gwarp; k < nt; k += 2 * nwarps) {
             const int t0 = batch_tile(b, k);
             const int t1 = k + nwarps < nt ? batch_tile(b, k + nwarps) : -1;
-            gr_pull_check(b, t0, t1, G + 1, L_GR0 + ((G + 1) & 1));
+            gr_pull_check(b, t0, t1, hlim, G + 1, L_GR0 + ((G + 1) & 1));
         }
         if (!grid_sync(b, 0)) return;
         if (timeline) ctl->gr_time[2] = gtimer();
@@ -1260,7 +1278,7 @@ __global__ void __launch_bounds__(NW * 32, solve_min_blocks<NW>()) k_solve(Batch
                 const long long c0 = clock64();
                 GrGeo g;
                 gr_prefetch(b, t, g, false);
-                gr_run(b, t, g, false, false, G + 1, L_GR0 + ((G + 1) & 1), sm.w.g[warp], sm.w.hs[warp], st);
+                gr_run(b, t, g, false, false, hlim, G + 1, L_GR0 + ((G + 1) & 1), sm.w.g[warp], sm.w.hs[warp], st);
                 if (lane == 0) {
                     const unsigned long long cyc = (unsigned long long)(clock64() - c0);
                     stat_add(st, ST_CYC_GR, cyc);
@@ -1336,11 +1354,18 @@ __global__ void __launch_bounds__(NW * 32, solve_min_blocks<NW>()) k_solve(Batch
             const unsigned long long total = *(volatile unsigned long long *)&ctl->total_active;
             for (int k = gtid; k < batch_nimg(b); k += nthreads) {
                 const int i = batch_img(b, k);
-                if (!b.ist[i].done && *(volatile unsigned long long *)&b.ist[i].active == 0) b.ist[i].done = 1;
+                // under a height limit an image without active pixels may still have
+                // some beyond it: the termination check decides
+                if (hlim == INF_H - 1 && !b.ist[i].done && *(volatile unsigned long long *)&b.ist[i].active == 0)
+                    b.ist[i].done = 1;
             }
             if (total == 0) {
-                finished = true;
-                break;
+                if (hlim == INF_H - 1) {
+                    finished = true;
+                    break;
+                }
+                full = true;  // nothing to push within the limit
+                continue;
             }
         }
         // ------------------------ checkerboard push rounds ------------------------
@@ -1365,7 +1390,7 @@ __global__ void __launch_bounds__(NW * 32, solve_min_blocks<NW>()) k_solve(Batch
                     // every thread has read it (push_tile's barriers come first)
                     const int idx = sm.p.idx;
                     if (idx >= n) break;
-                    push_tile(b, b.lists[(size_t)slot * b.list_cap + idx], prm, p, sm.p, st, &ctl->take[slot]);
+                    push_tile(b, b.lists[(size_t)slot * b.list_cap + idx], prm, hlim, p, sm.p, st, &ctl->take[slot]);
                 }
                 // the phase's tail: from the first block out of work to the barrier
                 if (threadIdx.x == 0) atomicMax(&ctl->push_idle[p & 1], ~gtimer());

@@ -131,12 +131,17 @@ struct SolveParams {
     int push_only;     // 1: sweeps only push; heights change only by exact local relabels
     // Diagnostic split of one solve into two launches, so that a profiler
     // sees the two main phases as separate kernels.  0: the whole solve.
-    // 1: initialisation, the first exact global relabel and its count pass,
+    // 1: initialisation, the first global relabel and its count pass,
     // then return (the work queues of the first push round stay in the
     // control block).  2: continue from the state a phase-1 launch left (the
     // control block not cleared in between): the push rounds of the first
     // outer iteration, then return.  A split leaves the solve unfinished.
     int phase;
+    // Height limit of the outer iterations: iteration k < near_outer relabels
+    // and pushes only where the distance to the sink is at most
+    // near_h * 4^k; later ones, and every one after an iteration with nothing
+    // to push, have no limit.
+    int near_h, near_outer;
     int warps;         // warps per block of the solver kernel (block shape 32 x warps over a 32x32 tile):
                        // 4, 8, 16 or 32; 0: by the solve's size (solve_warps)
 };
@@ -148,7 +153,7 @@ struct SolveParams {
 // for every case (4 rounds with 64 sweeps and a local relabel every 16 sweeps
 // took up to 2.9x longer on the 1920x1080 image with lambda 200).  The block
 // shape goes by the solve's size (solve_warps).
-constexpr SolveParams kDefaultSolveParams{64, 2, 24, 4, 0, 1 << 20, 0, 0, 0};
+constexpr SolveParams kDefaultSolveParams{66, 2, 24, 4, 0, 1 << 20, 0, 0, 9, 2, 0};
 
 // The block shape of a solve of n_tiles tiles: the shape asked for, or for 0
 // 32 x 16 up to 2048 tiles (a 1920x1080 image has 2040) and 32 x 8 above.
