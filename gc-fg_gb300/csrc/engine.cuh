@@ -147,13 +147,15 @@ struct SolveParams {
 };
 
 // Default solver settings of every entry point (before any tuning): 2 push
-// rounds per global relabel, 24 sweeps per tile visit, an exact local relabel
+// rounds per global relabel, 16 sweeps per tile visit, an exact local relabel
 // every 4 sweeps.  Measured on single images from 256x256 to 4096x4096 and on
 // the 256-image batch, these are at or near the fastest of the settings tried
-// for every case (4 rounds with 64 sweeps and a local relabel every 16 sweeps
-// took up to 2.9x longer on the 1920x1080 image with lambda 200).  The block
+// for every case.  24 sweeps, the default before the height limit, takes
+// longer where visits are hard: 1920x1080 with lambda 200 263 against 257 us,
+// 4096x4096 1136 against 1089, a 1024x768 graph with penalty 20 220 against
+// 201, the others the same; 12 and 8 are within 2% of 16 either way.  The block
 // shape goes by the solve's size (solve_warps).
-constexpr SolveParams kDefaultSolveParams{66, 2, 24, 4, 0, 1 << 20, 0, 0, 9, 2, 0};
+constexpr SolveParams kDefaultSolveParams{66, 2, 16, 4, 0, 1 << 20, 0, 0, 9, 2, 0};
 
 // The block shape of a solve of n_tiles tiles: the shape asked for, or for 0
 // 32 x 16 up to 2048 tiles (a 1920x1080 image has 2040) and 32 x 8 above.

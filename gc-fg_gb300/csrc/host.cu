@@ -1285,11 +1285,11 @@ gcfg_status gcfg_batch_autotune(gcfg_batch *b, int n, const int *widths, const i
     // sweeps between local relabels, blocks per SM, relabel-first, push-only.
     static const int c_warps[] = {4, 8, 16, 32};
     static const int c_push[] = {2, 4, 8, 16};
-    static const int c_sweeps[] = {16, 24, 32, 64, 128};
+    static const int c_sweeps[] = {16, 32, 64, 128};
     static const int c_bfs[] = {2, 4, 8, 16, 32};
     for (int pass = 0; pass < 2 && rc == GCFG_OK; ++pass) {
         for (int which = 0; which < 7 && rc == GCFG_OK; ++which) {
-            const int nc = which == 0 ? 4 : which == 1 ? 4 : which == 2 || which == 3 ? 5
+            const int nc = which == 0 || which == 1 || which == 2 ? 4 : which == 3 ? 5
                          : which == 4 ? per_sm_of(cur.warps) : 2;
             for (int c = 0; c < nc && rc == GCFG_OK; ++c) {
                 SolveParams p = cur;
