@@ -699,7 +699,7 @@ def tuned_vs_default(gcfg, stream, Ws, Hs, lams, d_rgb, d_scrib, offs, flows, sm
             "per_image": out, "results_equal": eq,
             "how": "each image as a batch of one through gcfg_batch_run; best of 5 device times (data term to cuts) "
                    "under the default settings (solver block by size: 32 x 16 up to 2048 tiles, else 32 x 8; 2 push "
-                   "rounds per global relabel, 24 sweeps, local relabel every 4) and under gcfg_batch_autotune's "
+                   "rounds per global relabel, 16 sweeps, local relabel every 4) and under gcfg_batch_autotune's "
                    "choice for that image"}
 
 

@@ -574,8 +574,9 @@ __device__ __forceinline__ void gr_prefetch(const Batch &b, int t, GrGeo &gg, bo
 // least current (distances only fall during a relabel), so no needed visit is
 // missed.  Distances above hlim are not passed on, so only heights up to hlim
 // are exact (hlim = INF_H - 1: all of them).
-__device__ void gr_run(const Batch &b, int t, const GrGeo &g, bool round0, bool direct, int hlim, int tag_next,
-                       int slot_next, GrScratch &sc, int *hs, unsigned long long *st) {
+// queue: whether it queues neighbours at all.
+__device__ void gr_run(const Batch &b, int t, const GrGeo &g, bool round0, bool direct, bool queue, int hlim,
+                       int tag_next, int slot_next, GrScratch &sc, int *hs, unsigned long long *st) {
     const int lane = threadIdx.x & 31;
     const size_t base = (size_t)t * TPX;
     unsigned m[6];
@@ -630,7 +631,7 @@ __device__ void gr_run(const Batch &b, int t, const GrGeo &g, bool round0, bool 
         own[HB_LFT + lane] = vl;
         own[HB_RGT + lane] = vr;
     }
-    if (!round0) {
+    if (queue) {
         const bool up_t = __any_sync(FULL, ((fu >> lane) & 1u) && vt < hlim && vt + 1 < ht);
         const bool up_b = __any_sync(FULL, ((fd >> lane) & 1u) && vb < hlim && vb + 1 < hb);
         const bool up_l = __any_sync(FULL, fl && vl < hlim && vl + 1 < hl);
@@ -643,16 +644,16 @@ __device__ void gr_run(const Batch &b, int t, const GrGeo &g, bool round0, bool 
     __syncwarp();
 }
 
-// After round 0 of a global relabel: tile t joins the first frontier round
-// when a neighbour's border, as round 0 left it, gives one of t's border
-// pixels (through its residual edge out of the tile) a shorter path than its
-// own round-0 distance.
+// After round 0 of a global relabel: tile t needs another visit (want) when a
+// neighbour's border, as round 0 left it, gives one of t's border pixels
+// (through its residual edge out of the tile) a shorter path than its own
+// round-0 distance.
 // Two tiles per call (t1 < 0: one), every load that depends only on the
 // tile issued first for both (image, neighbour table, own border lines and
 // masks), then the image's finished flag and the neighbours' border lines:
 // two memory round trips for the pair where one tile alone took four.  A
 // tile of a finished image is not checked.
-__device__ void gr_pull_check(const Batch &b, int t0, int t1, int hlim, int tag_next, int slot_next) {
+__device__ void gr_pull_check(const Batch &b, int t0, int t1, int hlim, bool want[2]) {
     const int lane = threadIdx.x & 31;
     const int tt[2] = {t0, t1 >= 0 ? t1 : t0};
     int img[2], ot[2], ob[2], ol[2], orr[2];
@@ -673,7 +674,6 @@ __device__ void gr_pull_check(const Batch &b, int t0, int t1, int hlim, int tag_
         rl[q] = mask_word(b, t, 0, lane) & 1u;
         rr[q] = mask_word(b, t, 1, lane) >> 31;
     }
-    bool want[2];
 #pragma unroll
     for (int q = 0; q < 2; ++q) {
         const int done = __ldcg(&b.ist[img[q]].done);
@@ -686,8 +686,7 @@ __device__ void gr_pull_check(const Batch &b, int t0, int t1, int hlim, int tag_
                          (rl[q] && hl < hlim && hl + 1 < ol[q]) || (rr[q] && hr < hlim && hr + 1 < orr[q]);
         want[q] = !done && __any_sync(FULL, imp);  // done is warp-uniform
     }
-    enqueue_warp(b, b.mark_gr, slot_next, tag_next, t0, lane == 0 && want[0]);
-    if (t1 >= 0) enqueue_warp(b, b.mark_gr, slot_next, tag_next, t1, lane == 0 && want[1]);
+    want[1] = want[1] && t1 >= 0;
 }
 // Source-side reachability closure of tile t given the halo's reach bits.
 __device__ void reach_tile(const Batch &b, int t, bool round0, int tag_next, int slot_next) {
@@ -1126,7 +1125,10 @@ __device__ __noinline__ int closure_check(const Batch &b, const SolveParams &prm
         const int img = __ldg(b.tile_img + t);
         if (vload(&b.ist[img].done)) continue;  // warp-uniform
         const unsigned live = __ldcg(b.hfin + (size_t)t * 32 + lane) & mask_word(b, t, 5, lane);
-        if (__any_sync(FULL, live != 0) && lane == 0) b.ist[img].active = 1;
+        if (__any_sync(FULL, live != 0) && lane == 0) {
+            b.ist[img].active = 1;
+            *(volatile int *)&ctl->open_images = 1;
+        }
     }
     for (int kb = gtid - lane; kb < nt; kb += nthreads) {  // warp-uniform
         const int k = kb + lane;
@@ -1151,17 +1153,17 @@ __device__ __noinline__ int closure_check(const Batch &b, const SolveParams &prm
         }
     }
     if (!grid_sync(b, 0)) return -1;
+    if (gtid == 0) ctl->closure_checks++;
+    if (vload(&ctl->open_images) == 0) {  // no image has an augmenting path left
+        if (gtid == 0) ctl->closure_ends++;
+        return 1;
+    }
     for (int k = gtid; k < batch_nimg(b); k += nthreads) {
         const int i = batch_img(b, k);
-        if (b.ist[i].done) continue;
-        if (*(volatile unsigned long long *)&b.ist[i].active == 0) b.ist[i].done = 1;
-        else atomicAdd(&ctl->open_images, 1);
+        if (!b.ist[i].done && *(volatile unsigned long long *)&b.ist[i].active == 0) b.ist[i].done = 1;
     }
-    if (gtid == 0) ctl->closure_checks++;
     if (!grid_sync(b, 0)) return -1;
-    if (vload(&ctl->open_images) != 0) return 0;
-    if (gtid == 0) ctl->closure_ends++;
-    return 1;
+    return 0;
 }
 
 // The block is NW warps over one 32x32 tile (thread block 32 x NW, the
@@ -1195,18 +1197,6 @@ __global__ void __launch_bounds__(NW * 32, solve_min_blocks<NW>()) k_solve(Batch
     PhaseClock clk;
     clk.start();
     const int nt = batch_ntiles(b);
-    if (prm.phase != 2) {
-        // fresh de-duplication marks and reach bits for this solve
-        for (int k = gtid; k < nt; k += nthreads) {
-            const int t = batch_tile(b, k);
-            b.mark_push[t] = -1;
-            b.mark_gr[t] = -1;
-        }
-        for (size_t i = gtid; i < (size_t)nt * 32; i += nthreads)
-            b.reach[(size_t)batch_tile(b, (int)(i >> 5)) * 32 + (i & 31)] = 0;
-        if (!grid_sync(b, 0)) return;
-        clk.charge(&ctl->t_init);
-    }
 
     int P = 0;  // push phase counter (even at the start of every outer iteration)
     int G = 0;  // global relabel round counter (tags of the tile frontier)
@@ -1244,10 +1234,16 @@ __global__ void __launch_bounds__(NW * 32, solve_min_blocks<NW>()) k_solve(Batch
             const int t = batch_tile(b, k);
             GrGeo g;
             gr_prefetch(b, t, g, true);
+            if (outer == 0) {
+                // fresh de-duplication marks and reach bits for this solve, which
+                // nothing reads before the next grid barrier
+                b.reach[(size_t)t * 32 + lane] = 0;
+                if (lane == 0) b.mark_push[t] = -1;
+                if (lane == 1) b.mark_gr[t] = -1;
+            }
             if (g.skip) continue;
             const long long c0 = clock64();
-            gr_run(b, t, g, true, nt >= 2 * nwarps, hlim, G + 1, L_GR0 + ((G + 1) & 1), sm.w.g[warp], sm.w.hs[warp],
-                   st);
+            gr_run(b, t, g, true, nt >= 2 * nwarps, false, hlim, 0, 0, sm.w.g[warp], sm.w.hs[warp], st);
             if (lane == 0) {
                 stat_add(st, ST_CYC_GR, (unsigned long long)(clock64() - c0));
                 stat_add(st, ST_GR_TILES, 1ull);
@@ -1258,12 +1254,47 @@ __global__ void __launch_bounds__(NW * 32, solve_min_blocks<NW>()) k_solve(Batch
         for (int k = gwarp; k < nt; k += 2 * nwarps) {
             const int t0 = batch_tile(b, k);
             const int t1 = k + nwarps < nt ? batch_tile(b, k + nwarps) : -1;
-            gr_pull_check(b, t0, t1, hlim, G + 1, L_GR0 + ((G + 1) & 1));
+            bool want[2];  // warp-uniform
+            gr_pull_check(b, t0, t1, hlim, want);
+            if (timeline && k == gwarp) ctl->gr_time[2] = gtimer();
+            if (hlim == INF_H - 1) {
+                enqueue_warp(b, b.mark_gr, L_GR0 + ((G + 1) & 1), G + 1, lane == 0 ? t0 : t1,
+                             lane < 2 && want[lane & 1]);
+                continue;
+            }
+            // Under a height limit one further visit takes the place of the
+            // frontier rounds, at once: its neighbours may be in theirs, so it
+            // may miss a path by way of a second tile, and some heights within
+            // the limit come out too high.  The push rounds then leave some
+            // excess to the next outer iteration; on the other hand a relabel
+            // takes two grid barriers, not three and one per frontier round
+            // (with this, no pass of its own to reset the marks, and one barrier
+            // less in the termination check: 256x256 160 -> 144 us on the device,
+            // 1920x1080 249 -> 230, 4096x4096 1190 -> 1130).
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                if (!want[q]) continue;
+                const int t = q ? t1 : t0;
+                const long long c0 = clock64();
+                GrGeo g;
+                gr_prefetch(b, t, g, false);
+                gr_run(b, t, g, false, false, false, hlim, 0, 0, sm.w.g[warp], sm.w.hs[warp], st);
+                if (lane == 0) {
+                    const unsigned long long cyc = (unsigned long long)(clock64() - c0);
+                    stat_add(st, ST_CYC_GR, cyc);
+                    stat_add(st, ST_GR_TILES, 1ull);
+                    if (prm.phase == 1) {  // the phase-split diagnostic only: shown as frontier round 0
+                        atomicAdd(&ctl->gr_front[0], 1);
+                        atomicMax(&ctl->gr_front_end[0], gtimer());
+                        atomicMax(&ctl->gr_front_maxcyc[0], cyc);
+                    }
+                }
+            }
         }
         if (!grid_sync(b, 0)) return;
-        if (timeline) ctl->gr_time[2] = gtimer();
+        if (timeline) ctl->gr_time[3] = gtimer();
         ++G;
-        for (int k = 1;; ++k) {
+        for (int k = 1; hlim == INF_H - 1; ++k) {
             const int slot = L_GR0 + (G & 1);
             const int n = vload(&ctl->size[slot]);
             if (n == 0) break;
@@ -1278,25 +1309,18 @@ __global__ void __launch_bounds__(NW * 32, solve_min_blocks<NW>()) k_solve(Batch
                 const long long c0 = clock64();
                 GrGeo g;
                 gr_prefetch(b, t, g, false);
-                gr_run(b, t, g, false, false, hlim, G + 1, L_GR0 + ((G + 1) & 1), sm.w.g[warp], sm.w.hs[warp], st);
+                gr_run(b, t, g, false, false, true, hlim, G + 1, L_GR0 + ((G + 1) & 1), sm.w.g[warp], sm.w.hs[warp],
+                       st);
                 if (lane == 0) {
-                    const unsigned long long cyc = (unsigned long long)(clock64() - c0);
-                    stat_add(st, ST_CYC_GR, cyc);
+                    stat_add(st, ST_CYC_GR, (unsigned long long)(clock64() - c0));
                     stat_add(st, ST_GR_TILES, 1ull);
-                    if (prm.phase == 1 && k <= GR_TIMELINE) {  // the phase-split diagnostic only
-                        atomicMax(&ctl->gr_front_end[k - 1], gtimer());
-                        atomicMax(&ctl->gr_front_maxcyc[k - 1], cyc);
-                    }
                 }
             }
             if (!grid_sync(b, 1u << slot)) return;
-            if (timeline && k <= GR_TIMELINE) {
-                ctl->gr_time[2 + k] = gtimer();
-                ctl->gr_front[k - 1] = n;
-            }
             ++G;
             if (gtid == 0) ctl->gr_rounds++;
         }
+        if (gtid == 0 && hlim < INF_H - 1 && (prm.phase != 1 || ctl->gr_front[0] > 0)) ctl->gr_rounds++;
         clk.charge(&ctl->t_gr);
         // ------------------------ count active nodes ------------------------
         // warp-uniform loop: the sums of a warp's tiles go out with one

@@ -61,11 +61,11 @@ struct Ctl {
     unsigned long long push_tiles, gr_tiles, reach_tiles;
     int gr_rounds, push_phases, reach_rounds, outer_iters;
     int global_relabels;
-    int open_images;     // images left open by the last termination check
+    int open_images;     // nonzero: the last termination check left an image open
     int closure_checks;  // termination checks by sink-side closure
     int closure_ends;    // solves that the closure check ended (no final global relabel)
     // device time per phase (ns, %globaltimer read by block 0 at barriers)
-    unsigned long long t_init, t_gr, t_count, t_push, t_reach;
+    unsigned long long t_gr, t_count, t_push, t_reach;
     unsigned long long push_sweeps, push_bfs;
     // SM cycles per section of the push visits, summed over visits
     unsigned long long cyc_load, cyc_bfs, cyc_sweep, cyc_wb, cyc_take;
@@ -77,10 +77,10 @@ struct Ctl {
     // keeps the earliest; t_push_tail sums (phase end - earliest idle)
     unsigned long long push_idle[2], t_push_tail;
     // timeline of the global relabel of a phase-1 launch (the phase-split
-    // diagnostic; %globaltimer ns, block 0 after each grid barrier):
-    // gr_time[0] its start, [1] after round 0, [2]
-    // after the pull check, [3 + k] after frontier round k (k < GR_TIMELINE);
-    // gr_front[k] the tiles of frontier round k
+    // diagnostic; %globaltimer ns of block 0): gr_time[0] its start, [1] after
+    // round 0, [2] after the first pull check, [3] after the second visits of
+    // the tiles whose check asked for one; gr_front[0] those tiles (the
+    // relabel runs under a height limit, so there is one such round)
     unsigned long long gr_time[3 + GR_TIMELINE];
     int gr_front[GR_TIMELINE];
     // per frontier round of that relabel: the latest end of a tile visit
