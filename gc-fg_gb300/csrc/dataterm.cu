@@ -114,12 +114,8 @@ __device__ __noinline__ int nlink_exact(int d2, double lambda, double s2) {
     return (int)round(lambda * exp(a));
 }
 
-// sigma^2 and 1 / (2 sigma^2) of each image, once per image.
-__global__ void k_img_params(const int *__restrict__ ilist, const ImgDesc *__restrict__ img, int n_img,
-                             ImgState *ist) {
-    const int li = blockIdx.x * blockDim.x + threadIdx.x;
-    if (li >= n_img) return;
-    const int im = ilist ? ilist[li] : li;
+// sigma^2 and the n-link constants of image im, from its sigma_sum.
+__device__ __forceinline__ void img_params(const ImgDesc *__restrict__ img, ImgState *ist, int im) {
     const unsigned long long s = ist[im].sigma_sum;
     const long long count = (long long)(img[im].W - 1) * img[im].H + (long long)img[im].W * (img[im].H - 1);
     const double s2 = (s == 0 || count == 0) ? 0.0 : (double)s / (double)count;
@@ -129,6 +125,14 @@ __global__ void k_img_params(const int *__restrict__ ilist, const ImgDesc *__res
     ist[im].const_w = (int)round(img[im].lambda);
     const double lam = img[im].lambda;
     ist[im].nl_margin = (float)(lam * (2.5e-7 * log(2.0 * lam + 1.0) + 1.5e-6) + 1e-6);
+}
+
+// The same for every image of a pass without scribbles (k_tlut_b otherwise
+// does it beside its tables: one launch and 3 us less per call).
+__global__ void k_img_params(const int *__restrict__ ilist, const ImgDesc *__restrict__ img, int n_img,
+                             ImgState *ist) {
+    const int li = blockIdx.x * blockDim.x + threadIdx.x;
+    if (li < n_img) img_params(img, ist, ilist ? ilist[li] : li);
 }
 
 __device__ __forceinline__ NlinkParams nlink_params(double lambda, const ImgState &st) {
@@ -276,7 +280,7 @@ __device__ __forceinline__ uint32_t sigma_chunk(uintptr_t lo, uintptr_t hi, uint
     return acc;
 }
 
-// One pass over a chunk of an image (CHUNK_PX consecutive pixels, row-major):
+// One pass over a chunk of an image (`chunk` consecutive pixels, row-major):
 // the exact sum of ||dI||^2 over right and down neighbour pairs (for sigma^2)
 // and the scribble colour histograms (privatised per block in shared memory,
 // equal bins of a warp aggregated with __match_any_sync before the shared
@@ -293,15 +297,15 @@ __device__ __forceinline__ uint32_t sigma_chunk(uintptr_t lo, uintptr_t hi, uint
 __global__ void __launch_bounds__(256, 8) k_hist_sigma_b(const uint8_t *__restrict__ rgb,
                                                       const uint8_t *__restrict__ scrib,
                                                       const ImgDesc *__restrict__ img,
-                                                      const int2 *__restrict__ chunk_map,
+                                                      const int2 *__restrict__ chunk_map, int chunk,
                                                       int *__restrict__ hist, ImgState *ist) {
     __shared__ uint4 keep[(3 * CHUNK_PX + 15) / 16 + 1];  // the chunk's bytes from its 16-aligned start
     const int2 cm = __ldg(chunk_map + blockIdx.x);  // (image, chunk within the image)
     const int im = cm.x;
     const int W = img[im].W, H = img[im].H;
     const long long npx = (long long)W * H;
-    const long long p0 = (long long)cm.y * CHUNK_PX;
-    const int n = (int)min((long long)CHUNK_PX, npx - p0);  // pixels of the chunk
+    const long long p0 = (long long)cm.y * chunk;
+    const int n = (int)min((long long)chunk, npx - p0);  // pixels of the chunk
     const long long pix0 = img[im].pix0;
     const uint8_t *base = rgb + 3 * pix0;
     const bool do_hist = scrib != nullptr;
@@ -338,81 +342,91 @@ __global__ void __launch_bounds__(256, 8) k_hist_sigma_b(const uint8_t *__restri
         __syncthreads();  // the kept colours
         const uint8_t *kb = reinterpret_cast<const uint8_t *>(keep) + (int)(((uintptr_t)base + 3 * p0) & 15);
         int *dst = hist + (size_t)im * 2 * NBINS;
-        // The chunk's scribble bytes, 16 per lane.  Scribbles come in short
-        // runs (strips, squares), so a lane's 16 bytes are often all marked
-        // while most lanes have none: the warp lists its marked bytes (a
-        // prefix sum of the lanes' counts) and bins them 32 per round, lane k
-        // taking item k of the list.  Equal bins of a round add once, with a
-        // fire-and-forget global add.
+        // The chunk's scribble bytes, one aligned word per lane (128 pixels per
+        // warp and step, so that a fully marked chunk is shared by all warps:
+        // with 16 bytes per lane and the list for every step, the border strip's
+        // chunks took the pass of a 256x256 image 17 us, of 1920x1080 20 us;
+        // 8.6 and 14.8 this way, launch included).
+        // Equal bins of a round add once, with a fire-and-forget global add.
+        // Where half the step's pixels are marked (rows of a strip), round j
+        // takes byte j of every lane; otherwise (ends of strips, squares) the
+        // warp lists its marked bytes by a prefix sum of the lanes' counts and
+        // bins them 32 per round, lane k taking item k of the list.
         const uintptr_t slo = (uintptr_t)(scrib + pix0), shi = slo + (uintptr_t)npx;
         const uintptr_t s0 = slo + (uintptr_t)p0;
-        const uintptr_t saw = s0 & ~(uintptr_t)15;
-        const int nsv = (int)((s0 + n - saw + 15) >> 4);
-        for (int v0 = (int)threadIdx.x - lane; v0 < nsv; v0 += blockDim.x) {
+        const uintptr_t saw = s0 & ~(uintptr_t)3;
+        const int nsw = (int)((s0 + n - saw + 3) >> 2);
+        auto bin = [&](bool on, int px, int cls) {  // pixel px of the chunk, class 1 or 2
+            int key = -1;
+            if (on) {
+                const uint32_t col = (uint32_t)kb[3 * px] | ((uint32_t)kb[3 * px + 1] << 8) |
+                                     ((uint32_t)kb[3 * px + 2] << 16);
+                key = (cls - 1) * NBINS + color_binw(col);
+            }
+            const unsigned same = __match_any_sync(0xffffffffu, key);
+            if (on && lane == __ffs(same) - 1) atomicAdd(dst + key, __popc(same));
+        };
+        for (int v0 = (int)threadIdx.x - lane; v0 < nsw; v0 += blockDim.x) {
             const int vi = v0 + lane;
-            const uintptr_t a = saw + 16 * (uintptr_t)vi;
-            const uint4 sv = vi < nsv ? vec_in(a, slo, shi) : make_uint4(0, 0, 0, 0);
-            const int o = (int)(a - s0);  // chunk pixel of the vector's byte 0
-            // bit b: byte b is 1 or 2 and lies in the chunk (4 bytes at a time:
-            // per-byte equality masks, then the bytes' top bits packed by a multiply)
+            const uintptr_t a = saw + 4 * (uintptr_t)vi;
+            const uint32_t w = vi < nsw ? word_in(a, slo, shi) : 0u;
+            const int o = (int)(a - s0);  // chunk pixel of the word's byte 0
+            // bit b: byte b is 1 or 2 and lies in the chunk
             unsigned todo = 0;
-            {
-                const uint32_t sw[4] = {sv.x, sv.y, sv.z, sv.w};
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    uint32_t m = __vcmpeq4(sw[j], 0x01010101u) | __vcmpeq4(sw[j], 0x02020202u);
-                    if (o < 0 || o + 16 > n) m &= byte_mask(o + 4 * j, 0, n);
-                    const uint32_t x = (m >> 7) & 0x01010101u;
-                    todo |= ((x * 0x01020408u) >> 24) << (4 * j);
-                }
+            for (int b = 0; b < 4; ++b) {
+                const uint32_t v = (w >> (8 * b)) & 0xFFu;
+                todo |= (unsigned)(v - 1u < 2u && o + b >= 0 && o + b < n) << b;
             }
             const int cnt = __popc(todo);
+            if (!__any_sync(0xffffffffu, cnt != 0)) continue;
+            const int total = (int)__reduce_add_sync(0xffffffffu, (unsigned)cnt);
+            if (total >= 64) {  // warp-uniform
+#pragma unroll
+                for (int b = 0; b < 4; ++b) bin((todo >> b) & 1u, o + b, (int)((w >> (8 * b)) & 0xFFu));
+                continue;
+            }
             int incl = cnt;  // inclusive prefix sum of the counts over the warp
 #pragma unroll
             for (int d = 1; d < 32; d <<= 1) {
                 const int v = __shfl_up_sync(0xffffffffu, incl, d);
                 if (lane >= d) incl += v;
             }
-            const int total = __shfl_sync(0xffffffffu, incl, 31);
             for (int r0 = 0; r0 < total; r0 += 32) {  // warp-uniform
                 const int k = r0 + lane;
                 // owner: the first lane whose inclusive sum exceeds k
-                int lo = 0;
+                int own = 0;
 #pragma unroll
                 for (int step = 16; step > 0; step >>= 1) {
-                    const int probe = __shfl_sync(0xffffffffu, incl, lo + step - 1);
-                    if (probe <= k) lo += step;
+                    const int probe = __shfl_sync(0xffffffffu, incl, own + step - 1);
+                    if (probe <= k) own += step;
                 }
-                const unsigned om = __shfl_sync(0xffffffffu, todo, lo);
-                const int oincl = __shfl_sync(0xffffffffu, incl, lo);
-                const int oo = __shfl_sync(0xffffffffu, o, lo);
-                const uint32_t w0 = __shfl_sync(0xffffffffu, sv.x, lo), w1 = __shfl_sync(0xffffffffu, sv.y, lo);
-                const uint32_t w2 = __shfl_sync(0xffffffffu, sv.z, lo), w3 = __shfl_sync(0xffffffffu, sv.w, lo);
-                int key = -1;
-                if (k < total) {
-                    // the (k - owner's exclusive sum)-th marked byte of the owner
-                    const int b = __fns(om, 0, k - (oincl - __popc(om)) + 1);
-                    const uint32_t wb = b < 8 ? (b < 4 ? w0 : w1) : (b < 12 ? w2 : w3);
-                    const int sc = (int)((wb >> (8 * (b & 3))) & 0xFFu);
-                    const int q = oo + b;  // pixel of the chunk
-                    const uint32_t col = (uint32_t)kb[3 * q] | ((uint32_t)kb[3 * q + 1] << 8) |
-                                         ((uint32_t)kb[3 * q + 2] << 16);
-                    key = (sc - 1) * NBINS + color_binw(col);
-                }
-                const unsigned same = __match_any_sync(0xffffffffu, key);
-                if (key >= 0 && lane == __ffs(same) - 1) atomicAdd(dst + key, __popc(same));
+                unsigned om = __shfl_sync(0xffffffffu, todo, own);
+                const int oincl = __shfl_sync(0xffffffffu, incl, own);
+                const int oo = __shfl_sync(0xffffffffu, o, own);
+                const uint32_t ow = __shfl_sync(0xffffffffu, w, own);
+                // the (k - owner's exclusive sum)-th of the owner's at most four marked bytes
+                const int skip = k - (oincl - __popc(om));
+#pragma unroll
+                for (int q = 0; q < 3; ++q)
+                    if (q < skip) om &= om - 1;
+                const int b = __ffs(om) - 1;
+                bin(k < total, oo + b, (int)((ow >> (8 * b)) & 0xFFu));
             }
         }
     }
     warp_atomic_add_u64(&ist[im].sigma_sum, acc);
 }
 
-// Per-bin t-link tables (one block per image, double precision).
+// Per-bin t-link tables (one block per image, double precision), and the
+// image's n-link constants by the block's last thread.
 __global__ void __launch_bounds__(1024) k_tlut_b(const int *__restrict__ ilist, const int *__restrict__ hist,
+                                                 const ImgDesc *__restrict__ img, ImgState *ist,
                                                  int *__restrict__ dp_lut, int *__restrict__ dn_lut,
                                                  double *raw_dp, double *raw_dn) {
     __shared__ long long part[2][32];
     const int im = ilist ? ilist[blockIdx.x] : blockIdx.x;
+    if (threadIdx.x == blockDim.x - 1) img_params(img, ist, im);
     const int *hf = hist + (size_t)im * 2 * NBINS;
     const int *hb = hf + NBINS;
     long long nf = 0, nb = 0;
@@ -756,21 +770,47 @@ __global__ void k_tlinks_apply(const uint8_t *__restrict__ rgb, long long n,
     dn[i] = __ldg(dn_lut + bin);
 }
 
-__global__ void k_nlinks_apply(const uint8_t *__restrict__ rgb, const ImgDesc *__restrict__ img,
-                               const ImgState *ist, int *__restrict__ up, int *__restrict__ down,
-                               int *__restrict__ left, int *__restrict__ right) {
+// One block per 32 x 32 pixels, thread (x, y) four rows of column x.  Each
+// edge is weighed once, by its left or upper pixel, which writes it to both
+// pixels' arrays; colours are read once per row, the right neighbour's and the
+// row below's come from the next lane and the next row.  (One thread per pixel
+// that weighed its four edges itself, and so each edge twice, from byte loads:
+// 17.3 us for 1279x853, 10.8 this way.)
+__global__ void __launch_bounds__(256) k_nlinks_apply(const uint8_t *__restrict__ rgb,
+                                                      const ImgDesc *__restrict__ img, const ImgState *ist,
+                                                      int *__restrict__ up, int *__restrict__ down,
+                                                      int *__restrict__ left, int *__restrict__ right) {
+    constexpr int ROWS = 4;
     const ImgDesc d = img[0];
     const int W = d.W, H = d.H;
-    const int x = blockIdx.x * blockDim.x + threadIdx.x;
-    const int y = blockIdx.y * blockDim.y + threadIdx.y;
-    if (x >= W || y >= H) return;
+    const int lane = threadIdx.x;
+    const int x = blockIdx.x * 32 + lane, y0 = (blockIdx.y * 8 + threadIdx.y) * ROWS;
     const NlinkParams q = nlink_params(d.lambda, ist[0]);
-    const long long i = (long long)y * W + x;
-    const uint8_t *p = rgb + 3 * i;
-    left[i] = x > 0 ? nlink_w(diff2p(p, p - 3), q) : 0;
-    right[i] = x + 1 < W ? nlink_w(diff2p(p, p + 3), q) : 0;
-    up[i] = y > 0 ? nlink_w(diff2p(p, p - 3 * (long long)W), q) : 0;
-    down[i] = y + 1 < H ? nlink_w(diff2p(p, p + 3 * (long long)W), q) : 0;
+    // colours of rows y0 .. y0 + ROWS, and of the pixel right of the last lane's
+    uint32_t c[ROWS + 1], cr[ROWS];
+#pragma unroll
+    for (int k = 0; k <= ROWS; ++k) {
+        const int y = y0 + k;
+        const uint8_t *p = rgb + 3 * ((long long)y * W + x);
+        c[k] = x < W && y < H ? pack_rgb(p) : 0u;
+        if (k < ROWS) cr[k] = lane == 31 && x + 1 < W && y < H ? pack_rgb(p + 3) : 0u;
+    }
+#pragma unroll
+    for (int k = 0; k < ROWS; ++k) {
+        const int y = y0 + k;
+        uint32_t r = __shfl_down_sync(0xffffffffu, c[k], 1);
+        if (lane == 31) r = cr[k];
+        if (x >= W || y >= H) continue;
+        const long long i = (long long)y * W + x;
+        const int wr = x + 1 < W ? nlink_w(diff2w(c[k], r), q) : 0;
+        const int wd = y + 1 < H ? nlink_w(diff2w(c[k], c[k + 1]), q) : 0;
+        right[i] = wr;
+        if (x + 1 < W) left[i + 1] = wr;
+        if (x == 0) left[i] = 0;
+        down[i] = wd;
+        if (y + 1 < H) up[i + W] = wd;
+        if (y == 0) up[i] = 0;
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -782,12 +822,15 @@ gcfg_status dt_tables(const DtArgs &a, cudaStream_t st) {
     // (with an image list the caller clears the histograms of those images)
     if (a.scrib && !a.ilist) GCFG_CK(cudaMemsetAsync(a.hist, 0, (size_t)a.n_img * 2 * NBINS * sizeof(int), st));
     GCFG_LAUNCH(GCFG_PK_HIST, st,
-                k_hist_sigma_b<<<a.total_chunks, 256, 0, st>>>(a.rgb, a.scrib, a.img, a.chunk_map, a.hist,
+                k_hist_sigma_b<<<a.total_chunks, 256, 0, st>>>(a.rgb, a.scrib, a.img, a.chunk_map, a.chunk, a.hist,
                                                                a.ist));
-    GCFG_LAUNCH(GCFG_PK_TLUT, st, k_img_params<<<div_up(a.n_img, 128), 128, 0, st>>>(a.ilist, a.img, a.n_img, a.ist));
     if (a.scrib)
         GCFG_LAUNCH(GCFG_PK_TLUT, st,
-                    k_tlut_b<<<a.n_img, 1024, 0, st>>>(a.ilist, a.hist, a.dp_lut, a.dn_lut, a.raw_dp, a.raw_dn));
+                    k_tlut_b<<<a.n_img, 1024, 0, st>>>(a.ilist, a.hist, a.img, a.ist, a.dp_lut, a.dn_lut, a.raw_dp,
+                                                       a.raw_dn));
+    else
+        GCFG_LAUNCH(GCFG_PK_TLUT, st,
+                    k_img_params<<<div_up(a.n_img, 128), 128, 0, st>>>(a.ilist, a.img, a.n_img, a.ist));
     GCFG_CK(cudaGetLastError());
     return GCFG_OK;
 }
@@ -808,7 +851,7 @@ gcfg_status dt_apply_tlinks(const DtArgs &a, long long n, int *dp, int *dn, cuda
 
 gcfg_status dt_apply_nlinks(const DtArgs &a, int W, int H, int *up, int *down, int *left, int *right,
                             cudaStream_t st) {
-    dim3 blk(32, 8), grd(div_up(W, 32), div_up(H, 8));
+    dim3 blk(32, 8), grd(div_up(W, 32), div_up(H, 32));
     GCFG_LAUNCH(GCFG_PK_OTHER, st,
                 k_nlinks_apply<<<grd, blk, 0, st>>>(a.rgb, a.img, a.ist, up, down, left, right));
     GCFG_CK(cudaGetLastError());

@@ -6,17 +6,21 @@
 namespace gcfg {
 
 constexpr int NBINS = 4096;                   // 16^3 colour bins per class
-#ifndef GCFG_CHUNK_PX
-// batch256 histogram/sigma pass: 0.159 / 0.128 / 0.118 / 0.143 ms at 2K / 4K / 8K / 16K pixels per
-// chunk; 8K leaves a single 1920x1080 image too few blocks (0.021 -> 0.032 ms), so 4K it is
-#define GCFG_CHUNK_PX 4096
-#endif
-constexpr int CHUNK_PX = GCFG_CHUNK_PX;       // pixels per block in per-image passes (about)
 
-// Rows of a W-wide image per block of the histogram / sigma pass.
-// Blocks of the per-image pass over an image: CHUNK_PX consecutive pixels
-// (row-major) each, the last one shorter.
-inline long long image_chunks(int W, int H) { return ((long long)W * H + CHUNK_PX - 1) / CHUNK_PX; }
+// Blocks of the per-image passes (histogram / sigma, extraction): each takes a
+// chunk of consecutive pixels (row-major) of one image, the image's last chunk
+// is shorter.  The chunk's size goes by the pixels of the whole pass: few
+// pixels make few blocks, and the pass then takes as long as one block.
+// Histogram / sigma pass at 1K / 2K / 4K pixels per chunk, one image (CUDA
+// events, launch included): 256x256 8.6 / 11.0 / 12.7 us, 900x900 12.2 / 11.3 /
+// 14.9, 1920x1080 16.4 / 14.8 / 16.8, 4096x4096 80 / 61 / 46; extraction
+// 6.1 / 6.1 / 6.1, 6.1 / 6.1 / 6.1, 8.2 / 7.2 / 6.5, 25 / 18 / 14.
+constexpr int CHUNK_PX = 4096;  // the largest chunk
+inline int chunk_px_for(long long px) { return px <= (1 << 18) ? 1024 : px <= (1 << 22) ? 2048 : CHUNK_PX; }
+// Chunks of any pass of at most n images and px pixels, whatever its own size
+// (a pass of fewer pixels may have smaller chunks).
+inline long long max_chunks(long long n, long long px) { return px / CHUNK_PX + (1 << 22) / 2048 + n + 1; }
+inline long long image_chunks(int W, int H, int chunk) { return ((long long)W * H + chunk - 1) / chunk; }
 
 // Device buffers of the data term for a batch (per image: 2*4096 histogram
 // bins, 4096 dp and dn entries).
@@ -29,6 +33,7 @@ struct DtArgs {
     const ImgDesc *img;
     ImgState *ist;
     const int2 *chunk_map;    // per chunk of the pass: (image index, chunk index within the image)
+    int chunk;                // pixels per chunk
     int *hist;
     int *dp_lut, *dn_lut;
     double *raw_dp, *raw_dn;  // optional (NULL): pre-rounding per-bin values

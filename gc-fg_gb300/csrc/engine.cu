@@ -39,7 +39,6 @@
 #include <cstring>
 #include <vector>
 
-#include "dataterm.cuh"  // CHUNK_PX: the data-term pass's chunks, reused by k_extract_rows
 #include "engine.cuh"
 
 namespace gcfg {
@@ -1554,7 +1553,7 @@ __global__ void __launch_bounds__(TILE_THREADS) k_extract(Batch b, uint8_t *smin
 }
 
 // The same cuts written row-major by output windows: block = one chunk of
-// an image (CHUNK_PX consecutive pixels, the data-term pass's chunk map),
+// an image (`chunk` consecutive pixels, the data-term pass's chunk map),
 // thread = one 16-byte window of the output arrays, aligned on the arrays'
 // addresses (smin and smax share their alignment mod 16).  A window takes
 // its bits from the row mask words of the tiles it covers, one row segment
@@ -1567,15 +1566,15 @@ __device__ __forceinline__ uint4 spread16(uint32_t bits) {
                       spread4((bits >> 12) & 15u));
 }
 
-__global__ void __launch_bounds__(256) k_extract_rows(Batch b, const int2 *__restrict__ chunk_map, uint8_t *smin,
-                                                      uint8_t *smax) {
+__global__ void __launch_bounds__(256) k_extract_rows(Batch b, const int2 *__restrict__ chunk_map, int chunk,
+                                                      uint8_t *smin, uint8_t *smax) {
     __shared__ long long s_row0;
     const int2 cm = __ldg(chunk_map + blockIdx.x);
     const int W = __ldg(&b.img[cm.x].W), H = __ldg(&b.img[cm.x].H);
     const int tile0 = __ldg(&b.img[cm.x].tile0), tiles_x = __ldg(&b.img[cm.x].tiles_x);
     const long long out0 = __ldg(&b.img[cm.x].out0);
     const long long npx = (long long)W * H;
-    const long long lo = (long long)cm.y * CHUNK_PX, hi = min(npx, lo + CHUNK_PX);  // the chunk's pixels
+    const long long lo = (long long)cm.y * chunk, hi = min(npx, lo + chunk);  // the chunk's pixels
     if (threadIdx.x == 0) s_row0 = lo / W;  // the chunk's first row
     __syncthreads();
     const long long row0 = s_row0;
@@ -1709,14 +1708,14 @@ gcfg_status launch_build_arrays(const Batch &b, const int *dp, const int *dn, in
     return GCFG_OK;
 }
 
-gcfg_status launch_extract_rows(const Batch &b, const int2 *chunk_map, long long n_chunks, uint8_t *smin,
-                               uint8_t *smax, cudaStream_t st) {
+gcfg_status launch_extract_rows(const Batch &b, const int2 *chunk_map, long long n_chunks, int chunk,
+                               uint8_t *smin, uint8_t *smax, cudaStream_t st) {
     if ((!smin && !smax) || n_chunks <= 0) return GCFG_OK;
     if (smin && smax && (((uintptr_t)smin ^ (uintptr_t)smax) & 15)) {
         // the windows need one alignment for both arrays: the tile-major kernel instead
         return launch_extract(b, smin, smax, nullptr, st);
     }
-    GCFG_LAUNCH(GCFG_PK_EXTRACT, st, k_extract_rows<<<(unsigned)n_chunks, 256, 0, st>>>(b, chunk_map, smin, smax));
+    GCFG_LAUNCH(GCFG_PK_EXTRACT, st, k_extract_rows<<<(unsigned)n_chunks, 256, 0, st>>>(b, chunk_map, chunk, smin, smax));
     GCFG_CK(cudaGetLastError());
     return GCFG_OK;
 }

@@ -46,6 +46,7 @@ struct Engine {
 
     int n_img = 0, n_tiles = 0;
     long long n_px = 0, total_chunks = 0;
+    int chunk = CHUNK_PX;  // pixels per chunk of the current layout
 
     // device
     ImgDesc *d_img = nullptr; size_t c_img = 0;
@@ -283,8 +284,7 @@ struct Engine {
     gcfg_status reserve_(int imgs, int tiles, long long px, bool dataterm, bool staging, bool arena) {
         GCFG_TRY(grow(d_img, c_img, imgs));
         GCFG_TRY(grow(d_ist, c_ist, imgs));
-        // chunks of the data-term pass: at most px / CHUNK_PX + one per image
-        const size_t chunks = (size_t)(px / CHUNK_PX) + (size_t)imgs + 1;
+        const size_t chunks = (size_t)max_chunks(imgs, px);
         GCFG_TRY(grow(d_cmap, c_cmap, chunks));
         GCFG_TRY(grow_host(h_cmap, ch_cmap, chunks));
         if (arena) {
@@ -337,6 +337,7 @@ struct Engine {
         count(n, W, H, tiles, px);
         if ((long long)tiles * TPX > (1LL << 40)) return GCFG_ERR_INVALID;
         GCFG_TRY(reserve(n, tiles, px, dataterm, staging, arena));
+        chunk = chunk_px_for(px);
         int t = 0;
         long long p = 0, ch = 0;
         for (int i = 0; i < n; ++i) {
@@ -355,7 +356,7 @@ struct Engine {
             h_chunk[i] = ch;
             t += d.n_tiles;
             p += (long long)W[i] * H[i];
-            ch += image_chunks(W[i], H[i]);
+            ch += image_chunks(W[i], H[i], chunk);
         }
         h_chunk[n] = ch;
         for (int i = 0; i < n; ++i)
@@ -467,6 +468,7 @@ struct Engine {
         a.img = d_img;
         a.ist = d_ist;
         a.chunk_map = d_cmap;
+        a.chunk = chunk;
         a.hist = d_hist;
         a.dp_lut = d_dpl;
         a.dn_lut = d_dnl;
@@ -762,7 +764,7 @@ static gcfg_status run_batch_eager(Engine &e, int n, const int *W, const int *H,
     GCFG_TRY(e.solve());
     uint8_t *dmin = staging ? (smin ? e.d_smin : nullptr) : smin;
     uint8_t *dmax = staging ? (smax ? e.d_smax : nullptr) : smax;
-    if (dmin || dmax) GCFG_TRY(launch_extract_rows(e.batch(), e.d_cmap, e.total_chunks, dmin, dmax, e.st));
+    if (dmin || dmax) GCFG_TRY(launch_extract_rows(e.batch(), e.d_cmap, e.total_chunks, e.chunk, dmin, dmax, e.st));
     if (staging) {
         if (smin) GCFG_CK(cudaMemcpyAsync(smin, e.d_smin, (size_t)e.n_px, cudaMemcpyDeviceToHost, e.st));
         if (smax) GCFG_CK(cudaMemcpyAsync(smax, e.d_smax, (size_t)e.n_px, cudaMemcpyDeviceToHost, e.st));
@@ -833,7 +835,7 @@ static gcfg_status graph_for(Engine &e, int n, const int *W, const int *H, const
             // graph must not hold it up on the copy engine
             if (rc == GCFG_OK) rc = e.readback();
             if (rc == GCFG_OK && (dmin || dmax))
-                rc = launch_extract_rows(e.batch(), e.d_cmap, e.total_chunks, dmin, dmax, e.st);
+                rc = launch_extract_rows(e.batch(), e.d_cmap, e.total_chunks, e.chunk, dmin, dmax, e.st);
             if (cudaStreamEndCapture(e.cap_st, &g) != cudaSuccess && rc == GCFG_OK) rc = GCFG_ERR_CUDA;
         }
         e.st = user;
@@ -959,7 +961,7 @@ static gcfg_status stage_extract(Engine &e, uint8_t *h_smin, uint8_t *h_smax, cu
     for (int g = 0; g < (int)e.groups.size(); ++g) {
         const Engine::Group &gr = e.groups[g];
         if (h_smin || h_smax)
-            GCFG_TRY(launch_extract_rows(e.batch(), e.d_cmap + gr.c0, gr.c1 - gr.c0, h_smin ? e.d_smin : nullptr,
+            GCFG_TRY(launch_extract_rows(e.batch(), e.d_cmap + gr.c0, gr.c1 - gr.c0, e.chunk, h_smin ? e.d_smin : nullptr,
                                          h_smax ? e.d_smax : nullptr, e.st));
         GCFG_CK(cudaEventRecord(e.ev_out[g], e.st));
         GCFG_CK(cudaStreamWaitEvent(out_st, e.ev_out[g], 0));
@@ -1059,7 +1061,7 @@ static gcfg_status submit_staged(Engine &e, Engine::Flight &f, int slot, int n, 
     // download is queued: behind it on the copy engine it would stall st
     GCFG_TRY(e.readback());
     if (h_smin || h_smax)
-        GCFG_TRY(launch_extract_rows(e.batch(), e.d_cmap, e.total_chunks, h_smin ? e.d_smin : nullptr,
+        GCFG_TRY(launch_extract_rows(e.batch(), e.d_cmap, e.total_chunks, e.chunk, h_smin ? e.d_smin : nullptr,
                                      h_smax ? e.d_smax : nullptr, e.st));
     GCFG_CK(cudaEventRecord(f.ev_ext, e.st));
     GCFG_CK(cudaStreamWaitEvent(e.dn_st, f.ev_ext, 0));

@@ -326,11 +326,13 @@ gcfg_status run_batch(Lane &L, std::vector<Req> &batch, const std::vector<Sessio
     cudaStream_t st = L.st;
     const int n = (int)batch.size();
     int nt = 0, nnew = 0, nedit = 0;
-    long long ch = 0;
+    long long ch = 0, batch_px = 0;
+    for (int k = 0; k < n; ++k) batch_px += (long long)snap[k].W * snap[k].H;
+    const int chunk = chunk_px_for(batch_px);
     for (int k = 0; k < n; ++k) {
         const Session &x = snap[k];
         L.h_il[k] = x.slot;
-        const long long nc = image_chunks(x.W, x.H);
+        const long long nc = image_chunks(x.W, x.H, chunk);
         for (long long c = 0; c < nc; ++c) L.h_cmap[ch + c] = make_int2(x.slot, (int)c);
         ch += nc;
         for (long long i = 0; i < x.n_tiles; ++i) {
@@ -389,6 +391,7 @@ gcfg_status run_batch(Lane &L, std::vector<Req> &batch, const std::vector<Sessio
     a.img = s.img;
     a.ist = s.ist;
     a.chunk_map = L.d_cmap;
+    a.chunk = chunk;
     a.hist = s.hist;
     a.dp_lut = s.dpl;
     a.dn_lut = s.dnl;
@@ -423,7 +426,7 @@ gcfg_status run_batch(Lane &L, std::vector<Req> &batch, const std::vector<Sessio
     prm.warps = solve_warps(prm.warps, nt);  // the lanes share the GPU in blocks of this shape
     GCFG_TRY(launch_solve(b, prm, nt, st,
                           s.cfg.lanes > 1 ? solve_grid_blocks(1 << 30, 0, prm.warps) / s.cfg.lanes : 0));
-    GCFG_TRY(launch_extract_rows(b, L.d_cmap, ch, s.smin, s.smax, st));
+    GCFG_TRY(launch_extract_rows(b, L.d_cmap, ch, chunk, s.smin, s.smax, st));
     for (int k = 0; k < n; ++k) {
         const Session &x = snap[k];
         const size_t npx = (size_t)x.W * x.H;
@@ -642,8 +645,8 @@ gcfg_status gcfg_serve_create(const gcfg_serve_config *cfg, gcfg_server **out) {
         chk(dalloc(L->d_tnew, LT)); chk(halloc(L->h_tnew, LT));
         chk(dalloc(L->d_tedit, LT)); chk(halloc(L->h_tedit, LT));
         chk(dalloc(L->d_il, LI)); chk(halloc(L->h_il, LI));
-        // chunks of a batch: at most its pixels / CHUNK_PX + one per image
-        chk(dalloc(L->d_cmap, LT * TPX / CHUNK_PX + LI + 1)); chk(halloc(L->h_cmap, LT * TPX / CHUNK_PX + LI + 1));
+        const size_t LC = (size_t)max_chunks((long long)LI, (long long)(LT * TPX));
+        chk(dalloc(L->d_cmap, LC)); chk(halloc(L->h_cmap, LC));
         chk(halloc(L->h_desc, LI)); chk(halloc(L->h_ist, LI));
         s->lanes.push_back(L);
     }
