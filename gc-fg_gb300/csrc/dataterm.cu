@@ -300,7 +300,8 @@ __global__ void __launch_bounds__(256, 8) k_hist_sigma_b(const uint8_t *__restri
                                                       const int2 *__restrict__ chunk_map, int chunk,
                                                       int *__restrict__ hist, ImgState *ist) {
     __shared__ uint4 keep[(3 * CHUNK_PX + 15) / 16 + 1];  // the chunk's bytes from its 16-aligned start
-    const int2 cm = __ldg(chunk_map + blockIdx.x);  // (image, chunk within the image)
+    // (image, chunk within the image); no map: one image
+    const int2 cm = chunk_map ? __ldg(chunk_map + blockIdx.x) : make_int2(0, (int)blockIdx.x);
     const int im = cm.x;
     const int W = img[im].W, H = img[im].H;
     const long long npx = (long long)W * H;
@@ -818,9 +819,8 @@ __global__ void __launch_bounds__(256) k_nlinks_apply(const uint8_t *__restrict_
 // ---------------------------------------------------------------------------
 
 gcfg_status dt_tables(const DtArgs &a, cudaStream_t st) {
-    // a.scrib == NULL: n-link tables only (the colour histograms need scribbles)
-    // (with an image list the caller clears the histograms of those images)
-    if (a.scrib && !a.ilist) GCFG_CK(cudaMemsetAsync(a.hist, 0, (size_t)a.n_img * 2 * NBINS * sizeof(int), st));
+    // a.scrib == NULL: n-link constants only (the colour histograms need
+    // scribbles); the caller has cleared the histograms
     GCFG_LAUNCH(GCFG_PK_HIST, st,
                 k_hist_sigma_b<<<a.total_chunks, 256, 0, st>>>(a.rgb, a.scrib, a.img, a.chunk_map, a.chunk, a.hist,
                                                                a.ist));

@@ -28,17 +28,18 @@ static gcfg_status grow(T *&p, size_t &cap, size_t need) {
     return GCFG_OK;
 }
 
-template <typename T>
-static gcfg_status grow_host(T *&p, size_t &cap, size_t need) {
-    if (need <= cap && p) return GCFG_OK;
-    if (p) cudaFreeHost(p);
-    p = nullptr;
-    cap = 0;
-    size_t n = need < 1 ? 1 : need;
-    if (cudaMallocHost(&p, n * sizeof(T)) != cudaSuccess) return GCFG_ERR_OOM;
-    cap = n;
-    return GCFG_OK;
-}
+// Carves arrays out of one allocation, each 256-byte aligned; with a null
+// base it only measures.
+struct Carver {
+    char *base;
+    size_t off = 0;
+    template <typename T>
+    void put(T *&p, size_t n) {
+        off = (off + 255) & ~size_t(255);
+        p = base ? reinterpret_cast<T *>(base + off) : nullptr;
+        off += n * sizeof(T);
+    }
+};
 
 struct Engine {
     cudaStream_t st = nullptr;
@@ -48,41 +49,51 @@ struct Engine {
     long long n_px = 0, total_chunks = 0;
     int chunk = CHUNK_PX;  // pixels per chunk of the current layout
 
-    // device
-    ImgDesc *d_img = nullptr; size_t c_img = 0;
-    ImgState *d_ist = nullptr; size_t c_ist = 0;
-    int2 *d_cmap = nullptr; size_t c_cmap = 0;  // per chunk of the data-term pass: (image, chunk in image)
-    int *d_tile_img = nullptr; size_t c_timg = 0;
-    int4 *d_cap = nullptr; size_t c_cap = 0;
-    int *d_exc = nullptr; size_t c_exc = 0;
-    int *d_h = nullptr; size_t c_h = 0;
-    int *d_hb = nullptr; size_t c_hb = 0;
-    int4 *d_tnb = nullptr; size_t c_tnb = 0;
-    unsigned *d_hfin = nullptr; size_t c_hfin = 0;
-    unsigned *d_reach = nullptr; size_t c_reach = 0;
-    unsigned *d_tmask = nullptr; size_t c_tmask = 0;
-    int *d_tact = nullptr; size_t c_tact = 0;
-    unsigned long long *d_tpos = nullptr; size_t c_tpos = 0;
-    int *d_lists = nullptr; size_t c_lists = 0; int list_cap = 0;
-    int *d_mpush = nullptr; size_t c_mpush = 0;
-    int *d_mgr = nullptr; size_t c_mgr = 0;
-    Ctl *d_ctl = nullptr; size_t c_ctl = 0;
-    int *d_hist = nullptr; size_t c_hist = 0;
-    int *d_dpl = nullptr; size_t c_dpl = 0;
-    int *d_dnl = nullptr; size_t c_dnl = 0;
-    double *d_raw = nullptr; size_t c_raw = 0;
+    // Device arrays, carved out of one allocation (slab) for up to cap_imgs
+    // images, cap_chunks chunks and cap_tiles tiles: an allocation costs about
+    // 35 us and its release 30 (measured), whatever its size, so a graph that
+    // is made for one solve pays for one.  What a run clears comes first
+    // (control block, per-image states, histograms), in that order, then what
+    // it uploads (descriptors, chunk map, tile owners).
+    char *slab = nullptr;
+    size_t cap_imgs = 0, cap_chunks = 0, cap_tiles = 0;
+    bool cap_dt = false;       // with histograms and t-link tables
+    size_t want_label = 0;     // int32 labels beside the arena (graph API)
+    Ctl *d_ctl = nullptr;
+    ImgState *d_ist = nullptr;
+    int *d_hist = nullptr;
+    ImgDesc *d_img = nullptr;
+    int2 *d_cmap = nullptr;    // per chunk of the data-term pass: (image, chunk in image)
+    int *d_tile_img = nullptr;
+    int *d_dpl = nullptr, *d_dnl = nullptr;
+    int4 *d_cap = nullptr;
+    int *d_exc = nullptr, *d_h = nullptr, *d_hb = nullptr;
+    int4 *d_tnb = nullptr;
+    unsigned *d_hfin = nullptr, *d_reach = nullptr, *d_tmask = nullptr;
+    int *d_tact = nullptr;
+    unsigned long long *d_tpos = nullptr;
+    int *d_lists = nullptr; int list_cap = 0;
+    int *d_mpush = nullptr, *d_mgr = nullptr;
+    int32_t *d_label = nullptr;
+    bool ctl_clean = false;    // the control block is zero
     // staging for host entry points
     uint8_t *d_rgb = nullptr; size_t c_rgb = 0;
     uint8_t *d_scrib = nullptr; size_t c_scrib = 0;
     uint8_t *d_smin = nullptr; size_t c_smin = 0;
     uint8_t *d_smax = nullptr; size_t c_smax = 0;
-    // host (pinned)
-    ImgDesc *h_img = nullptr; size_t ch_img = 0;
-    ImgState *h_ist = nullptr; size_t ch_ist = 0;
-    long long *h_chunk = nullptr; size_t ch_chunk = 0;  // first chunk of each image
-    int2 *h_cmap = nullptr; size_t ch_cmap = 0;
-    int *h_tile_img = nullptr; size_t ch_timg = 0;
-    Ctl *h_ctl = nullptr; size_t ch_ctl = 0;
+    // Host mirrors of the control block and states (read back) and of the
+    // uploaded tables, in one allocation with the device's offsets: pinned, or
+    // ordinary memory for the graph API, whose copies are small and blocking
+    // anyway (pinned memory costs about 100 us to allocate and 150 to release)
+    bool pinned = true;
+    char *h_slab = nullptr;
+    size_t h_imgs = 0, h_chunks = 0, h_tiles = 0;  // its capacities
+    Ctl *h_ctl = nullptr;
+    ImgState *h_ist = nullptr;
+    ImgDesc *h_img = nullptr;
+    int2 *h_cmap = nullptr;
+    int *h_tile_img = nullptr;
+    std::vector<long long> h_chunk;  // first chunk of each image
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
 
     int max_grid = 0;  // solver blocks (0: as many as fit, capped at half the tiles)
@@ -130,12 +141,13 @@ struct Engine {
     // the two batches stays ordered on st; their uploads (cp_st) and
     // downloads (dn_st) overlap the other batch's compute.
     struct RunSet {
-        ImgDesc *h_img = nullptr; size_t ch_img = 0;
-        ImgState *h_ist = nullptr; size_t ch_ist = 0;
-        long long *h_chunk = nullptr; size_t ch_chunk = 0;
-        int2 *h_cmap = nullptr; size_t ch_cmap = 0;
-        int *h_tile_img = nullptr; size_t ch_timg = 0;
-        Ctl *h_ctl = nullptr; size_t ch_ctl = 0;
+        char *h_slab = nullptr;
+        size_t h_imgs = 0, h_chunks = 0, h_tiles = 0;
+        Ctl *h_ctl = nullptr;
+        ImgState *h_ist = nullptr;
+        ImgDesc *h_img = nullptr;
+        int2 *h_cmap = nullptr;
+        int *h_tile_img = nullptr;
         uint8_t *d_rgb = nullptr; size_t c_rgb = 0;
         uint8_t *d_scrib = nullptr; size_t c_scrib = 0;
         uint8_t *d_smin = nullptr; size_t c_smin = 0;
@@ -159,12 +171,10 @@ struct Engine {
     bool in_flight() const { return flight[0].busy || flight[1].busy; }
 
     void swap_set(RunSet &o) {
-        std::swap(h_img, o.h_img); std::swap(ch_img, o.ch_img);
-        std::swap(h_ist, o.h_ist); std::swap(ch_ist, o.ch_ist);
-        std::swap(h_chunk, o.h_chunk); std::swap(ch_chunk, o.ch_chunk);
-        std::swap(h_tile_img, o.h_tile_img); std::swap(ch_timg, o.ch_timg);
-        std::swap(h_cmap, o.h_cmap); std::swap(ch_cmap, o.ch_cmap);
-        std::swap(h_ctl, o.h_ctl); std::swap(ch_ctl, o.ch_ctl);
+        std::swap(h_slab, o.h_slab);
+        std::swap(h_imgs, o.h_imgs); std::swap(h_chunks, o.h_chunks); std::swap(h_tiles, o.h_tiles);
+        std::swap(h_ctl, o.h_ctl); std::swap(h_ist, o.h_ist); std::swap(h_img, o.h_img);
+        std::swap(h_cmap, o.h_cmap); std::swap(h_tile_img, o.h_tile_img);
         std::swap(d_rgb, o.d_rgb); std::swap(c_rgb, o.c_rgb);
         std::swap(d_scrib, o.d_scrib); std::swap(c_scrib, o.c_scrib);
         std::swap(d_smin, o.d_smin); std::swap(c_smin, o.c_smin);
@@ -173,12 +183,7 @@ struct Engine {
     }
 
     static void free_set(RunSet &o) {
-        if (o.h_img) cudaFreeHost(o.h_img);
-        if (o.h_ist) cudaFreeHost(o.h_ist);
-        if (o.h_chunk) cudaFreeHost(o.h_chunk);
-        if (o.h_tile_img) cudaFreeHost(o.h_tile_img);
-        if (o.h_cmap) cudaFreeHost(o.h_cmap);
-        if (o.h_ctl) cudaFreeHost(o.h_ctl);
+        if (o.h_slab) cudaFreeHost(o.h_slab);  // (a handle with two sets has pinned ones)
         cudaFree(o.d_rgb); cudaFree(o.d_scrib); cudaFree(o.d_smin); cudaFree(o.d_smax);
         if (o.ev0) cudaEventDestroy(o.ev0);
         if (o.ev1) cudaEventDestroy(o.ev1);
@@ -195,7 +200,7 @@ struct Engine {
     bool laid_out(int n, const int *W, const int *H, const double *lam) const {
         if ((int)lay_w.size() != n) return false;
         for (int i = 0; i < n; ++i)
-            if (lay_w[i] != W[i] || lay_h[i] != H[i] || lay_lam[i] != lam[i]) return false;
+            if (lay_w[i] != W[i] || lay_h[i] != H[i] || lay_lam[i] != (lam ? lam[i] : 0.0)) return false;
         return true;
     }
 
@@ -209,19 +214,9 @@ struct Engine {
         }
         if (dn_st) cudaStreamDestroy(dn_st);
         dn_st = nullptr;
-        cudaFree(d_img); cudaFree(d_ist); cudaFree(d_cmap); cudaFree(d_tile_img);
-        cudaFree(d_cap); cudaFree(d_exc); cudaFree(d_h); cudaFree(d_hb); cudaFree(d_tnb); cudaFree(d_hfin); cudaFree(d_reach);
-        cudaFree(d_tmask); cudaFree(d_tact); cudaFree(d_tpos);
-        cudaFree(d_lists);
-        cudaFree(d_mpush); cudaFree(d_mgr); cudaFree(d_ctl);
-        cudaFree(d_hist); cudaFree(d_dpl); cudaFree(d_dnl); cudaFree(d_raw);
+        cudaFree(slab);
         cudaFree(d_rgb); cudaFree(d_scrib); cudaFree(d_smin); cudaFree(d_smax);
-        if (h_img) cudaFreeHost(h_img);
-        if (h_ist) cudaFreeHost(h_ist);
-        if (h_chunk) cudaFreeHost(h_chunk);
-        if (h_cmap) cudaFreeHost(h_cmap);
-        if (h_tile_img) cudaFreeHost(h_tile_img);
-        if (h_ctl) cudaFreeHost(h_ctl);
+        free_host();
         if (ev0) cudaEventDestroy(ev0);
         if (ev1) cudaEventDestroy(ev1);
         drop_graphs();
@@ -238,22 +233,16 @@ struct Engine {
         ev_mark = nullptr;
         cudaFree(d_iota);
         d_iota = nullptr;
-        d_img = nullptr; d_ist = nullptr; d_cmap = nullptr; d_tile_img = nullptr;
-        d_cap = nullptr; d_exc = nullptr; d_h = nullptr; d_hb = nullptr; d_tnb = nullptr; d_hfin = nullptr; d_reach = nullptr;
-        d_tmask = nullptr; d_tact = nullptr; d_tpos = nullptr;
-        d_lists = nullptr;
-        d_mpush = d_mgr = nullptr; d_ctl = nullptr;
-        d_hist = d_dpl = d_dnl = nullptr; d_raw = nullptr;
+        slab = nullptr;
+        cap_imgs = cap_chunks = cap_tiles = 0;
+        carve_device(nullptr);
         d_rgb = d_scrib = d_smin = d_smax = nullptr;
-        h_img = nullptr; h_ist = nullptr; h_chunk = nullptr; h_cmap = nullptr; h_tile_img = nullptr; h_ctl = nullptr;
         ev0 = ev1 = nullptr;
     }
 
     gcfg_status init() {
         GCFG_CK(cudaEventCreate(&ev0));
         GCFG_CK(cudaEventCreate(&ev1));
-        GCFG_TRY(grow(d_ctl, c_ctl, 1));
-        GCFG_TRY(grow_host(h_ctl, ch_ctl, 1));
         return GCFG_OK;
     }
 
@@ -267,53 +256,103 @@ struct Engine {
         }
     }
 
-    std::vector<const void *> buffers() const {
-        return {d_img, d_ist, d_cmap, d_tile_img, d_cap, d_exc, d_h, d_hb, d_tnb, d_hfin, d_reach, d_tmask, d_tact, d_tpos,
-                d_lists, d_mpush, d_mgr, d_ctl, d_hist, d_dpl, d_dnl, d_rgb, d_scrib, d_smin, d_smax,
-                h_img, h_ist, h_chunk, h_cmap, h_tile_img, h_ctl};
+    // Device pointers for the current capacities; returns the slab's size.
+    size_t carve_device(char *base) {
+        Carver c{base};
+        const size_t T = cap_tiles;
+        c.put(d_ctl, 1);
+        c.put(d_ist, cap_imgs);
+        c.put(d_hist, cap_dt ? cap_imgs * 2 * NBINS : 0);
+        c.put(d_img, cap_imgs);
+        c.put(d_cmap, cap_chunks);
+        c.put(d_tile_img, T);
+        c.put(d_dpl, cap_dt ? cap_imgs * NBINS : 0);
+        c.put(d_dnl, cap_dt ? cap_imgs * NBINS : 0);
+        c.put(d_cap, T * TPX);
+        c.put(d_exc, T * TPX);
+        c.put(d_h, T * TPX);
+        c.put(d_hb, T * 4 * 32);
+        c.put(d_tnb, T);
+        c.put(d_hfin, T * 32);
+        c.put(d_reach, T * 32);
+        c.put(d_tmask, T * 6 * 32);
+        c.put(d_tact, T);
+        c.put(d_tpos, T);
+        c.put(d_lists, (size_t)L_NLISTS * T);
+        c.put(d_mpush, T);
+        c.put(d_mgr, T);
+        c.put(d_label, want_label);
+        list_cap = (int)T;
+        return c.off;
     }
 
+    // Host mirrors for the given capacities (the device's offsets up to the
+    // histograms' place, and from the descriptors on).
+    size_t carve_host(char *base) {
+        Carver c{base};
+        c.put(h_ctl, 1);
+        c.put(h_ist, h_imgs);
+        c.put(h_img, h_imgs);
+        c.put(h_cmap, h_chunks);
+        c.put(h_tile_img, h_tiles);
+        return c.off;
+    }
+
+    void free_host() {
+        if (pinned) {
+            if (h_slab) cudaFreeHost(h_slab);
+        } else {
+            free(h_slab);
+        }
+        h_slab = nullptr;
+        h_imgs = h_chunks = h_tiles = 0;
+        carve_host(nullptr);
+    }
+
+    std::vector<const void *> buffers() const { return {slab, h_slab, d_rgb, d_scrib, d_smin, d_smax}; }
+
     // Grow the buffers; any reallocation invalidates the captured graphs.
-    gcfg_status reserve(int imgs, int tiles, long long px, bool dataterm, bool staging, bool arena = true) {
+    gcfg_status reserve(int imgs, int tiles, long long px, bool dataterm, bool staging) {
         const std::vector<const void *> before = buffers();
-        const gcfg_status rc = reserve_(imgs, tiles, px, dataterm, staging, arena);
+        const gcfg_status rc = reserve_(imgs, tiles, px, dataterm, staging);
         if (buffers() != before) ++alloc_gen;
         return rc;
     }
 
-    gcfg_status reserve_(int imgs, int tiles, long long px, bool dataterm, bool staging, bool arena) {
-        GCFG_TRY(grow(d_img, c_img, imgs));
-        GCFG_TRY(grow(d_ist, c_ist, imgs));
+    gcfg_status reserve_(int imgs, int tiles, long long px, bool dataterm, bool staging) {
         const size_t chunks = (size_t)max_chunks(imgs, px);
-        GCFG_TRY(grow(d_cmap, c_cmap, chunks));
-        GCFG_TRY(grow_host(h_cmap, ch_cmap, chunks));
-        if (arena) {
-            GCFG_TRY(grow(d_tile_img, c_timg, tiles));
-            GCFG_TRY(grow(d_cap, c_cap, (size_t)tiles * TPX));
-            GCFG_TRY(grow(d_exc, c_exc, (size_t)tiles * TPX));
-            GCFG_TRY(grow(d_h, c_h, (size_t)tiles * TPX));
-            GCFG_TRY(grow(d_hb, c_hb, (size_t)tiles * 4 * 32));
-            GCFG_TRY(grow(d_tnb, c_tnb, (size_t)tiles));
-            GCFG_TRY(grow(d_hfin, c_hfin, (size_t)tiles * 32));
-            GCFG_TRY(grow(d_reach, c_reach, (size_t)tiles * 32));
-            GCFG_TRY(grow(d_tmask, c_tmask, (size_t)tiles * 6 * 32));
-            GCFG_TRY(grow(d_tact, c_tact, tiles));
-            GCFG_TRY(grow(d_tpos, c_tpos, tiles));
-            if ((size_t)tiles > (size_t)list_cap || !d_lists) {
-                GCFG_TRY(grow(d_lists, c_lists, (size_t)L_NLISTS * tiles));
-                list_cap = tiles;
+        if (!slab || (size_t)imgs > cap_imgs || chunks > cap_chunks || (size_t)tiles > cap_tiles ||
+            (dataterm && !cap_dt)) {
+            cudaFree(slab);
+            slab = nullptr;
+            lay_w.clear();  // nothing is laid out any more
+            if ((size_t)imgs > cap_imgs) cap_imgs = imgs;
+            if (chunks > cap_chunks) cap_chunks = chunks;
+            if ((size_t)tiles > cap_tiles) cap_tiles = tiles;
+            cap_dt = cap_dt || dataterm;
+            if (cudaMalloc(&slab, carve_device(nullptr)) != cudaSuccess) {
+                cudaGetLastError();
+                slab = nullptr;
+                cap_imgs = cap_chunks = cap_tiles = 0;
+                cap_dt = false;
+                carve_device(nullptr);
+                return GCFG_ERR_OOM;
             }
-            GCFG_TRY(grow(d_mpush, c_mpush, tiles));
-            GCFG_TRY(grow(d_mgr, c_mgr, tiles));
+            carve_device(slab);
         }
-        GCFG_TRY(grow_host(h_img, ch_img, imgs));
-        GCFG_TRY(grow_host(h_ist, ch_ist, imgs));
-        GCFG_TRY(grow_host(h_chunk, ch_chunk, (size_t)imgs + 1));
-        if (arena) GCFG_TRY(grow_host(h_tile_img, ch_timg, tiles));
-        if (dataterm) {
-            GCFG_TRY(grow(d_hist, c_hist, (size_t)imgs * 2 * NBINS));
-            GCFG_TRY(grow(d_dpl, c_dpl, (size_t)imgs * NBINS));
-            GCFG_TRY(grow(d_dnl, c_dnl, (size_t)imgs * NBINS));
+        if (!h_slab || h_imgs != cap_imgs || h_chunks != cap_chunks || h_tiles != cap_tiles) {
+            free_host();
+            h_imgs = cap_imgs;
+            h_chunks = cap_chunks;
+            h_tiles = cap_tiles;
+            const size_t bytes = carve_host(nullptr);
+            if (pinned ? cudaMallocHost(&h_slab, bytes) != cudaSuccess
+                       : (h_slab = static_cast<char *>(malloc(bytes))) == nullptr) {
+                h_slab = nullptr;
+                free_host();
+                return GCFG_ERR_OOM;
+            }
+            carve_host(h_slab);
         }
         if (staging) {
             GCFG_TRY(grow(d_rgb, c_rgb, (size_t)px * 3));
@@ -324,9 +363,20 @@ struct Engine {
         return GCFG_OK;
     }
 
+    // Clear what every run starts from zero: control block, per-image states
+    // and, with a data term, histograms (they lie next to each other).
+    gcfg_status zero(int n) {
+        char *end = cap_dt ? reinterpret_cast<char *>(d_hist + (size_t)n * 2 * NBINS)
+                           : reinterpret_cast<char *>(d_ist + n);
+        GCFG_CK(cudaMemsetAsync(d_ctl, 0, (size_t)(end - reinterpret_cast<char *>(d_ctl)), st));
+        ctl_clean = true;
+        return GCFG_OK;
+    }
+
     // Lay out a batch: descriptors, tile -> image map, chunk offsets; upload.
-    gcfg_status layout(int n, const int *W, const int *H, const double *lam, bool dataterm, bool staging,
-                       bool arena = true) {
+    // A layout that is on the device already (same sizes and lambdas) is not
+    // uploaded again.
+    gcfg_status layout(int n, const int *W, const int *H, const double *lam, bool dataterm, bool staging) {
         if (n < 1) return GCFG_ERR_INVALID;
         for (int i = 0; i < n; ++i) {
             if (W[i] < 1 || H[i] < 1 || (long long)W[i] * H[i] > (1LL << 31) - 1) return GCFG_ERR_INVALID;
@@ -336,47 +386,55 @@ struct Engine {
         long long px;
         count(n, W, H, tiles, px);
         if ((long long)tiles * TPX > (1LL << 40)) return GCFG_ERR_INVALID;
-        GCFG_TRY(reserve(n, tiles, px, dataterm, staging, arena));
+        GCFG_TRY(reserve(n, tiles, px, dataterm, staging));
         chunk = chunk_px_for(px);
-        int t = 0;
-        long long p = 0, ch = 0;
-        for (int i = 0; i < n; ++i) {
-            ImgDesc &d = h_img[i];
-            d.W = W[i];
-            d.H = H[i];
-            d.tiles_x = div_up(W[i], TILE_W);
-            d.tiles_y = div_up(H[i], TILE_H);
-            d.tile0 = t;
-            d.n_tiles = d.tiles_x * d.tiles_y;
-            d.pix0 = p;
-            d.lambda = lam ? lam[i] : 0.0;
-            d.out0 = p;
-            if (arena)
-                for (int k = 0; k < d.n_tiles; ++k) h_tile_img[t + k] = i;
-            h_chunk[i] = ch;
-            t += d.n_tiles;
-            p += (long long)W[i] * H[i];
-            ch += image_chunks(W[i], H[i], chunk);
-        }
-        h_chunk[n] = ch;
-        for (int i = 0; i < n; ++i)
-            for (long long c = h_chunk[i]; c < h_chunk[i + 1]; ++c) h_cmap[c] = make_int2(i, (int)(c - h_chunk[i]));
         n_img = n;
-        n_tiles = t;
-        n_px = p;
-        total_chunks = ch;
-        GCFG_CK(cudaMemcpyAsync(d_img, h_img, n * sizeof(ImgDesc), cudaMemcpyHostToDevice, st));
-        GCFG_CK(cudaMemcpyAsync(d_cmap, h_cmap, (size_t)ch * sizeof(int2), cudaMemcpyHostToDevice, st));
-        if (arena)
-            GCFG_CK(cudaMemcpyAsync(d_tile_img, h_tile_img, (size_t)t * sizeof(int), cudaMemcpyHostToDevice, st));
-        GCFG_CK(cudaMemsetAsync(d_ist, 0, n * sizeof(ImgState), st));
-        lay_w.assign(W, W + n);
-        lay_h.assign(H, H + n);
-        if (lam)
-            lay_lam.assign(lam, lam + n);
-        else
-            lay_lam.assign(n, 0.0);
-        return GCFG_OK;
+        n_tiles = tiles;
+        n_px = px;
+        h_chunk.resize((size_t)n + 1);
+        h_chunk[0] = 0;
+        for (int i = 0; i < n; ++i) h_chunk[i + 1] = h_chunk[i] + image_chunks(W[i], H[i], chunk);
+        total_chunks = h_chunk[n];
+        if (!laid_out(n, W, H, lam)) {
+            lay_w.clear();  // until the upload is queued
+            int t = 0;
+            long long p = 0;
+            for (int i = 0; i < n; ++i) {
+                ImgDesc &d = h_img[i];
+                d.W = W[i];
+                d.H = H[i];
+                d.tiles_x = div_up(W[i], TILE_W);
+                d.tiles_y = div_up(H[i], TILE_H);
+                d.tile0 = t;
+                d.n_tiles = d.tiles_x * d.tiles_y;
+                d.pix0 = p;
+                d.lambda = lam ? lam[i] : 0.0;
+                d.out0 = p;
+                for (int k = 0; k < d.n_tiles; ++k) h_tile_img[t + k] = i;
+                for (long long c = h_chunk[i]; c < h_chunk[i + 1]; ++c) h_cmap[c] = make_int2(i, (int)(c - h_chunk[i]));
+                t += d.n_tiles;
+                p += (long long)W[i] * H[i];
+            }
+            // the three tables in one copy, gaps included, unless the gaps are
+            // most of it (a small layout in a handle made for a large one)
+            const size_t b_img = n * sizeof(ImgDesc), b_cmap = (size_t)total_chunks * sizeof(int2),
+                         b_timg = (size_t)t * sizeof(int);
+            const size_t span = (size_t)(reinterpret_cast<char *>(d_tile_img) - reinterpret_cast<char *>(d_img)) + b_timg;
+            if (span <= 2 * (b_img + b_cmap + b_timg) + (64 << 10)) {
+                GCFG_CK(cudaMemcpyAsync(d_img, h_img, span, cudaMemcpyHostToDevice, st));
+            } else {
+                GCFG_CK(cudaMemcpyAsync(d_img, h_img, b_img, cudaMemcpyHostToDevice, st));
+                GCFG_CK(cudaMemcpyAsync(d_cmap, h_cmap, b_cmap, cudaMemcpyHostToDevice, st));
+                GCFG_CK(cudaMemcpyAsync(d_tile_img, h_tile_img, b_timg, cudaMemcpyHostToDevice, st));
+            }
+            lay_w.assign(W, W + n);
+            lay_h.assign(H, H + n);
+            if (lam)
+                lay_lam.assign(lam, lam + n);
+            else
+                lay_lam.assign(n, 0.0);
+        }
+        return zero(n);
     }
 
     // Split the laid-out batch into up to MAX_GROUPS groups of consecutive
@@ -484,14 +542,15 @@ struct Engine {
     }
 
     gcfg_status solve() {
-        GCFG_CK(cudaMemsetAsync(d_ctl, 0, sizeof(Ctl), st));
+        if (!ctl_clean) GCFG_CK(cudaMemsetAsync(d_ctl, 0, sizeof(Ctl), st));
+        ctl_clean = false;
         return launch_solve(batch(), prm, n_tiles, st, max_grid);
     }
 
     // Queue the read-back of the per-image states and the control block.
     gcfg_status readback() {
-        GCFG_CK(cudaMemcpyAsync(h_ist, d_ist, n_img * sizeof(ImgState), cudaMemcpyDeviceToHost, st));
-        GCFG_CK(cudaMemcpyAsync(h_ctl, d_ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, st));
+        const size_t bytes = (size_t)(reinterpret_cast<char *>(d_ist + n_img) - reinterpret_cast<char *>(d_ctl));
+        GCFG_CK(cudaMemcpyAsync(h_ctl, d_ctl, bytes, cudaMemcpyDeviceToHost, st));
         return GCFG_OK;
     }
 
@@ -560,7 +619,6 @@ struct gcfg_graph {
     bool varying = false;
     bool built = false;
     bool solved = false;
-    int32_t *d_label = nullptr;
 };
 
 struct gcfg_segmenter {
@@ -606,8 +664,7 @@ gcfg_status gcfg_set_graph(gcfg_graph *g) {
     if (!g) return GCFG_ERR_INVALID;
     if (!g->dp || !g->dn) return GCFG_ERR_STATE;
     Engine &e = g->e;
-    GCFG_CK(cudaMemsetAsync(e.d_ist, 0, sizeof(ImgState), e.st));
-    GCFG_CK(cudaMemsetAsync(e.d_ctl, 0, sizeof(Ctl), e.st));
+    GCFG_TRY(e.zero(1));
     GCFG_TRY(launch_build_arrays(e.batch(), g->dp, g->dn, g->penalty, g->varying ? g->up : nullptr, g->down,
                                  g->left, g->right, e.st));
     GCFG_TRY(e.fetch());
@@ -625,17 +682,16 @@ gcfg_status gcfg_init(int w, int h, const int32_t *dp, const int32_t *dn, int32_
     g->W = w;
     g->H = h;
     g->penalty = penalty;
+    g->e.pinned = false;
+    g->e.want_label = (size_t)w * h;
     gcfg_status rc = g->e.init();
     if (rc == GCFG_OK) rc = g->e.layout(1, &w, &h, nullptr, false, false);
-    if (rc == GCFG_OK && cudaMalloc(&g->d_label, (size_t)w * h * sizeof(int32_t)) != cudaSuccess)
-        rc = GCFG_ERR_OOM;
     if (rc == GCFG_OK && dp) {
         gcfg_set_dataterms(g, dp, dn);
         if (up) rc = gcfg_set_edges(g, up, down, left, right);
         if (rc == GCFG_OK) rc = gcfg_set_graph(g);
     }
     if (rc) {
-        cudaFree(g->d_label);
         delete g;
         return rc;
     }
@@ -663,7 +719,11 @@ gcfg_status gcfg_optimize(gcfg_graph *g, int32_t *host_label, gcfg_result *res) 
     GCFG_CK(cudaEventRecord(e.ev0, e.st));
     GCFG_TRY(e.solve());
     GCFG_CK(cudaEventRecord(e.ev1, e.st));
-    if (host_label) GCFG_TRY(launch_extract(e.batch(), nullptr, nullptr, g->d_label, e.st));
+    if (host_label) {
+        GCFG_TRY(launch_extract(e.batch(), nullptr, nullptr, e.d_label, e.st));
+        GCFG_CK(cudaMemcpyAsync(host_label, e.d_label, (size_t)g->W * g->H * sizeof(int32_t), cudaMemcpyDeviceToHost,
+                                e.st));
+    }
     GCFG_TRY(e.fetch());
     // the graph is consumed in place, as in the reference: re-solving needs
     // gcfg_set_graph again (GraphCut.cu:385-534 leaves the residual graph)
@@ -672,13 +732,7 @@ gcfg_status gcfg_optimize(gcfg_graph *g, int32_t *host_label, gcfg_result *res) 
     float ms = 0.f;
     cudaEventElapsedTime(&ms, e.ev0, e.ev1);
     if (res) e.result(0, res, ms);
-    GCFG_TRY(e.status());
-    if (host_label) {
-        GCFG_CK(cudaMemcpyAsync(host_label, g->d_label, (size_t)g->W * g->H * sizeof(int32_t),
-                                cudaMemcpyDeviceToHost, e.st));
-        GCFG_CK(cudaStreamSynchronize(e.st));
-    }
-    return GCFG_OK;
+    return e.status();
 }
 
 gcfg_status gcfg_get_cuts(gcfg_graph *g, uint8_t *d_smin, uint8_t *d_smax) {
@@ -691,7 +745,6 @@ gcfg_status gcfg_get_cuts(gcfg_graph *g, uint8_t *d_smin, uint8_t *d_smax) {
 
 gcfg_status gcfg_end(gcfg_graph *g) {
     if (!g) return GCFG_ERR_INVALID;
-    cudaFree(g->d_label);
     delete g;
     return GCFG_OK;
 }
@@ -700,47 +753,92 @@ gcfg_status gcfg_end(gcfg_graph *g) {
 // Stand-alone data term and n-links (one image)
 // ---------------------------------------------------------------------------
 
-static gcfg_status one_image_tables(Engine &e, const uint8_t *rgb, const uint8_t *scrib, int w, int h,
-                                    double lambda, double *raw_dp, double *raw_dn, DtArgs &a) {
-    GCFG_TRY(e.init());
-    GCFG_TRY(e.layout(1, &w, &h, &lambda, true, false, false));
-    a = e.dt(rgb, scrib);
-    if (raw_dp || raw_dn) {
-        GCFG_TRY(grow(e.d_raw, e.c_raw, 2 * NBINS));
-        a.raw_dp = e.d_raw;
-        a.raw_dn = e.d_raw + NBINS;
+namespace {
+
+// Tables of one image: everything in one device allocation, released on return.
+struct OneImage {
+    char *slab = nullptr;
+    ImgState *ist = nullptr;
+    int *hist = nullptr, *dpl = nullptr, *dnl = nullptr;
+    ImgDesc *img = nullptr;
+    double *raw = nullptr;
+    ImgDesc desc;  // the host's copy: alive until the stream is synchronised
+    ~OneImage() { cudaFree(slab); }
+
+    size_t carve(char *base, bool with_hist, bool with_raw) {
+        Carver c{base};
+        c.put(ist, 1);
+        c.put(hist, with_hist ? 2 * NBINS : 0);
+        c.put(img, 1);
+        c.put(dpl, with_hist ? NBINS : 0);
+        c.put(dnl, with_hist ? NBINS : 0);
+        c.put(raw, with_raw ? 2 * NBINS : 0);
+        return c.off;
     }
-    return dt_tables(a, e.st);
-}
+
+    gcfg_status tables(const uint8_t *rgb, const uint8_t *scrib, int w, int h, double lambda, bool with_raw,
+                       cudaStream_t st, DtArgs &a) {
+        const bool with_hist = scrib != nullptr;
+        if (cudaMalloc(&slab, carve(nullptr, with_hist, with_raw)) != cudaSuccess) {
+            cudaGetLastError();
+            slab = nullptr;
+            return GCFG_ERR_OOM;
+        }
+        carve(slab, with_hist, with_raw);
+        memset(&desc, 0, sizeof(desc));
+        desc.W = w;
+        desc.H = h;
+        desc.lambda = lambda;
+        GCFG_CK(cudaMemcpyAsync(img, &desc, sizeof(desc), cudaMemcpyHostToDevice, st));
+        GCFG_CK(cudaMemsetAsync(ist, 0, (size_t)(reinterpret_cast<char *>(img) - reinterpret_cast<char *>(ist)), st));
+        memset(&a, 0, sizeof(a));
+        a.n_img = 1;
+        a.chunk = chunk_px_for((long long)w * h);
+        a.total_chunks = image_chunks(w, h, a.chunk);
+        a.rgb = rgb;
+        a.scrib = scrib;
+        a.img = img;
+        a.ist = ist;
+        a.hist = hist;
+        a.dp_lut = dpl;
+        a.dn_lut = dnl;
+        a.raw_dp = with_raw ? raw : nullptr;
+        a.raw_dn = with_raw ? raw + NBINS : nullptr;
+        return dt_tables(a, st);
+    }
+};
+
+}  // namespace
 
 gcfg_status gcfg_tlinks(const uint8_t *d_rgb, const uint8_t *d_scrib, int n, int32_t *d_dp, int32_t *d_dn,
                         double *h_raw_dp, double *h_raw_dn, void *stream) {
     if (!d_rgb || !d_scrib || !d_dp || !d_dn || n <= 0) return GCFG_ERR_INVALID;
-    Engine e;
-    e.st = (cudaStream_t)stream;
+    cudaStream_t st = (cudaStream_t)stream;
+    OneImage o;
     DtArgs a;
     // the image is treated as n x 1: histograms and tables need no geometry
-    GCFG_TRY(one_image_tables(e, d_rgb, d_scrib, n, 1, 0.0, h_raw_dp, h_raw_dn, a));
-    GCFG_TRY(dt_apply_tlinks(a, n, d_dp, d_dn, e.st));
+    GCFG_TRY(o.tables(d_rgb, d_scrib, n, 1, 0.0, h_raw_dp || h_raw_dn, st, a));
+    GCFG_TRY(dt_apply_tlinks(a, n, d_dp, d_dn, st));
     if (h_raw_dp)
-        GCFG_CK(cudaMemcpyAsync(h_raw_dp, a.raw_dp, NBINS * sizeof(double), cudaMemcpyDeviceToHost, e.st));
+        GCFG_CK(cudaMemcpyAsync(h_raw_dp, a.raw_dp, NBINS * sizeof(double), cudaMemcpyDeviceToHost, st));
     if (h_raw_dn)
-        GCFG_CK(cudaMemcpyAsync(h_raw_dn, a.raw_dn, NBINS * sizeof(double), cudaMemcpyDeviceToHost, e.st));
-    GCFG_CK(cudaStreamSynchronize(e.st));
+        GCFG_CK(cudaMemcpyAsync(h_raw_dn, a.raw_dn, NBINS * sizeof(double), cudaMemcpyDeviceToHost, st));
+    GCFG_CK(cudaStreamSynchronize(st));
     return GCFG_OK;
 }
 
 gcfg_status gcfg_nlinks(const uint8_t *d_rgb, int w, int h, double lambda, int32_t *d_up, int32_t *d_down,
                         int32_t *d_left, int32_t *d_right, void *stream) {
     if (!d_rgb || !d_up || !d_down || !d_left || !d_right || w <= 0 || h <= 0) return GCFG_ERR_INVALID;
+    if ((long long)w * h > (1LL << 31) - 1) return GCFG_ERR_INVALID;
     if (!(lambda >= 0) || lambda * 1.0000001 + 1 > (double)GCFG_MAX_CAP) return GCFG_ERR_INVALID;
-    Engine e;
-    e.st = (cudaStream_t)stream;
+    cudaStream_t st = (cudaStream_t)stream;
+    OneImage o;
     DtArgs a;
-    // no scribbles: the colour tables are skipped, only the n-link table is made
-    GCFG_TRY(one_image_tables(e, d_rgb, nullptr, w, h, lambda, nullptr, nullptr, a));
-    GCFG_TRY(dt_apply_nlinks(a, w, h, d_up, d_down, d_left, d_right, e.st));
-    GCFG_CK(cudaStreamSynchronize(e.st));
+    // no scribbles: the colour tables are skipped, only the n-link constants are made
+    GCFG_TRY(o.tables(d_rgb, nullptr, w, h, lambda, false, st, a));
+    GCFG_TRY(dt_apply_nlinks(a, w, h, d_up, d_down, d_left, d_right, st));
+    GCFG_CK(cudaStreamSynchronize(st));
     return GCFG_OK;
 }
 
@@ -828,7 +926,7 @@ static gcfg_status graph_for(Engine &e, int n, const int *W, const int *H, const
         if (cudaStreamBeginCapture(e.cap_st, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
             rc = GCFG_ERR_CUDA;
         } else {
-            if (cudaMemsetAsync(e.d_ist, 0, (size_t)n * sizeof(ImgState), e.st) != cudaSuccess) rc = GCFG_ERR_CUDA;
+            rc = e.zero(n);
             if (rc == GCFG_OK) rc = e.build_images(drgb, dscrib);
             if (rc == GCFG_OK) rc = e.solve();
             // the state read-back first: a label download queued after the
@@ -946,8 +1044,6 @@ static gcfg_status stage_build(Engine &e) {
         a.ilist = e.d_iota + gr.i0;
         a.total_chunks = gr.c1 - gr.c0;
         a.chunk_map = e.d_cmap + gr.c0;
-        GCFG_CK(cudaMemsetAsync(e.d_hist + (size_t)gr.i0 * 2 * NBINS, 0,
-                                (size_t)(gr.i1 - gr.i0) * 2 * NBINS * sizeof(int), e.st));
         GCFG_TRY(dt_tables(a, e.st));
         Batch b = e.batch();
         b.tlist = e.d_iota + gr.t0;
@@ -1015,7 +1111,6 @@ static gcfg_status run_batch_staged(Engine &e, int n, const int *W, const int *H
 static gcfg_status submit_staged(Engine &e, Engine::Flight &f, int slot, int n, const int *W, const int *H,
                                  const double *lam, const uint8_t *h_rgb, const uint8_t *h_scrib, uint8_t *h_smin,
                                  uint8_t *h_smax) {
-    GCFG_TRY(grow_host(e.h_ctl, e.ch_ctl, 1));
     if (!e.ev0) GCFG_CK(cudaEventCreate(&e.ev0));
     if (!e.ev1) GCFG_CK(cudaEventCreate(&e.ev1));
     if (!e.cp_st) GCFG_CK(cudaStreamCreateWithFlags(&e.cp_st, cudaStreamNonBlocking));
