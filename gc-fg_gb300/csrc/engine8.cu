@@ -8,9 +8,8 @@
 // d (0 left, 1 right, 2 up, 3 down, 4 up-left, 5 up-right, 6 down-left,
 // 7 down-right).  One cooperative launch runs the whole solve:
 //   * exact global relabel: the distances to the sink-connected pixels
-//     (excess < 0) over the residual edges, by Bellman-Ford rounds over
-//     32x32 tiles, each tile relaxed to its fixpoint in shared memory
-//     (gr8_tile);
+//     (excess < 0) over the residual edges, by rounds over 32x32 tiles with a
+//     bit-parallel BFS of each tile (gr8_tile);
 //   * count: pixels with excess that can still reach the sink; none left
 //     after an exact global relabel means the preflow is maximum (an exact
 //     termination test);
@@ -48,6 +47,8 @@ struct G8 {
     long long n;
     int *cap;  // 8 * n
     int *e, *h, *mark;
+    unsigned *tm;  // NPLANE x 32 row masks per 32x32 tile, made by each global relabel
+    int *due;      // per 32x8 tile: the last tile round that has to visit it
     Ctl8 *ctl;
 };
 
@@ -55,6 +56,7 @@ struct P8 {
     int max_outer;   // global relabels at most
     int rounds;      // tile rounds between global relabels
     int sweeps;      // push/relabel sweeps per tile visit
+    int near_h;      // > 0: the first iteration relabels and pushes only this close to the sinks (engine.cuh, near_h)
 };
 
 enum { E8_BARRIER = 1, E8_OUTER = 2 };
@@ -150,8 +152,9 @@ __global__ void k8_build(G8 g, const int *__restrict__ dp, const int *__restrict
 // capacities, excess and heights and a one-pixel ring of heights (corners
 // included) are staged in shared memory, up to `sweeps` push/relabel sweeps
 // run with block barriers only, and the results go back as additive deltas.
-// A tile without a pixel that has excess and a finite height is left after
-// reading its excess and heights (returns false).
+// A visit that ends with a pixel still active makes its tile due in the next
+// round, and flow that leaves the tile makes the receiving one due; a round
+// visits the tiles that are due.
 // Every tile of the image is visited concurrently in a round, so a tile's
 // ring heights are a snapshot and its neighbours change its pixels meanwhile;
 // that stays safe because every concurrent update is an addition: a pixel's
@@ -164,190 +167,367 @@ __global__ void k8_build(G8 g, const int *__restrict__ dp, const int *__restrict
 // decide termination.
 constexpr int T8W = 32, T8H = 8;
 #ifndef GCFG_N8_ROUNDS
-#define GCFG_N8_ROUNDS 12   // tile rounds between global relabels
+#define GCFG_N8_ROUNDS 8    // tile rounds between global relabels
 #endif
 #ifndef GCFG_N8_SWEEPS
 #define GCFG_N8_SWEEPS 8    // sweeps per tile visit
 #endif
-__device__ bool tile8_visit(const G8 &g, int t, int tiles_x, int sweeps) {
+__device__ __forceinline__ void red_shared_if(int *p, int v) {  // *p += v, nothing when v is 0
+    const unsigned a = (unsigned)__cvta_generic_to_shared(p);
+    asm volatile("{\n .reg .pred q;\n setp.ne.s32 q, %1, 0;\n @q red.shared.add.s32 [%0], %1;\n}" ::"r"(a), "r"(v)
+                 : "memory");
+}
+
+__device__ void tile8_visit(const G8 &g, int t, int tiles_x, int sweeps, int hlim, int round) {
+    // excess and capacities have a ring too: flow that leaves the tile collects
+    // there (a ring cell's excess, and its capacity back into the tile)
     __shared__ int sh[T8H + 2][T8W + 2];
-    __shared__ int se[T8H][T8W];
-    __shared__ int sc[ND][T8H][T8W];
+    __shared__ int se[T8H + 2][T8W + 2];
+    __shared__ int sc[ND][T8H + 2][T8W + 2];
+    __shared__ int live[3];
     const int lx = threadIdx.x & 31, ly = threadIdx.x >> 5;
     const int x = (t % tiles_x) * T8W + lx, y = (t / tiles_x) * T8H + ly;
     const bool inb = x < g.W && y < g.H;
     const long long i = (long long)y * g.W + x;
-    const int e0 = inb ? g.e[i] : 0;
-    int hh = inb ? g.h[i] : INF_H;
-    if (!__syncthreads_or(e0 > 0 && hh < INF_H)) return false;  // nothing to push here
+    const int e0 = inb ? __ldcg(g.e + i) : 0;
+    int hh = inb ? __ldcg(g.h + i) : INF_H;
     int c0[ND];
 #pragma unroll
-    for (int d = 0; d < ND; ++d) {
-        c0[d] = inb ? g.cap[(long long)d * g.n + i] : 0;
-        sc[d][ly][lx] = c0[d];
+    for (int d = 0; d < ND; ++d) c0[d] = inb ? __ldcg(g.cap + (long long)d * g.n + i) : 0;
+    // this thread's ring cell, if it has one: the rows above and below (with
+    // the corners), then the sides
+    constexpr int RING = 2 * (T8W + 2) + 2 * T8H;
+    int rx = -1, ry = 0;
+    if (threadIdx.x < 2 * (T8W + 2)) {
+        rx = threadIdx.x % (T8W + 2);
+        ry = threadIdx.x < T8W + 2 ? 0 : T8H + 1;
+    } else if (threadIdx.x < RING) {
+        rx = (threadIdx.x - 2 * (T8W + 2)) & 1 ? T8W + 1 : 0;
+        ry = 1 + ((threadIdx.x - 2 * (T8W + 2)) >> 1);
     }
-    se[ly][lx] = e0;
-    auto hat = [&](int xx, int yy) -> int {
-        return xx >= 0 && yy >= 0 && xx < g.W && yy < g.H ? g.h[(long long)yy * g.W + xx] : INF_H;
-    };
+    static_assert(RING <= 256, "a ring cell per thread");
+    if (rx >= 0) {
+        const int xx = x - lx + rx - 1, yy = y - ly + ry - 1;
+        const bool in = xx >= 0 && yy >= 0 && xx < g.W && yy < g.H;
+        sh[ry][rx] = in ? __ldcg(g.h + (long long)yy * g.W + xx) : INF_H;
+        se[ry][rx] = 0;
+#pragma unroll
+        for (int d = 0; d < ND; ++d) sc[d][ry][rx] = 0;
+    }
+#pragma unroll
+    for (int d = 0; d < ND; ++d) sc[d][ly + 1][lx + 1] = c0[d];
+    se[ly + 1][lx + 1] = e0;
+    if (threadIdx.x < 3) live[threadIdx.x] = 0;
     sh[ly + 1][lx + 1] = hh;
-    if (ly == 0) sh[0][lx + 1] = hat(x, y - 1);
-    if (ly == T8H - 1) sh[T8H + 1][lx + 1] = hat(x, y + 1);
-    if (lx == 0) sh[ly + 1][0] = hat(x - 1, y);
-    if (lx == T8W - 1) sh[ly + 1][T8W + 1] = hat(x + 1, y);
-    if (lx == 0 && ly == 0) sh[0][0] = hat(x - 1, y - 1);
-    if (lx == T8W - 1 && ly == 0) sh[0][T8W + 1] = hat(x + 1, y - 1);
-    if (lx == 0 && ly == T8H - 1) sh[T8H + 1][0] = hat(x - 1, y + 1);
-    if (lx == T8W - 1 && ly == T8H - 1) sh[T8H + 1][T8W + 1] = hat(x + 1, y + 1);
+    bool alive = true;
     __syncthreads();
     for (int s = 0; s < sweeps; ++s) {
-        // push half: heights fixed
-        bool pushed = false;
-        int e = se[ly][lx];
-        if (e > 0 && hh < INF_H) {
+        // push half: heights fixed.  All loads first, the flows in registers,
+        // then fire-and-forget atomics.
+        int e = *(volatile int *)&se[ly + 1][lx + 1];
+        int hn[ND];
+        const bool on = e > 0 && hh <= hlim;
+        if (on) {
+            int cd[ND], f[ND];
+#pragma unroll
+            for (int d = 0; d < ND; ++d) {
+                cd[d] = sc[d][ly + 1][lx + 1];
+                hn[d] = sh[ly + 1 + dyd(d)][lx + 1 + dxd(d)];
+            }
             const int e_in = e;
 #pragma unroll
             for (int d = 0; d < ND; ++d) {
-                const int dx = dxd(d), dy = dyd(d);
-                const int cd = sc[d][ly][lx];
-                if (e <= 0 || cd <= 0 || sh[ly + 1 + dy][lx + 1 + dx] != hh - 1) continue;
-                const int f = min(e, cd);
-                sc[d][ly][lx] = cd - f;
-                e -= f;
-                const int nx = lx + dx, ny = ly + dy;
-                if (nx >= 0 && ny >= 0 && nx < T8W && ny < T8H) {
-                    atomicAdd(&se[ny][nx], f);
-                    atomicAdd(&sc[opp(d)][ny][nx], f);
-                } else {
-                    const long long j = (long long)(y + dy) * g.W + (x + dx);
-                    atomicAdd(&g.e[j], f);
-                    atomicAdd(&g.cap[(long long)opp(d) * g.n + j], f);
-                }
+                f[d] = hn[d] == hh - 1 ? min(e, cd[d]) : 0;
+                e -= f[d];
             }
             if (e != e_in) {
-                atomicSub(&se[ly][lx], e_in - e);
-                pushed = true;
+#pragma unroll
+                for (int d = 0; d < ND; ++d) {
+                    const int ny = ly + 1 + dyd(d), nx = lx + 1 + dxd(d);
+                    if (f[d]) sc[d][ly + 1][lx + 1] = cd[d] - f[d];
+                    red_shared_if(&se[ny][nx], f[d]);
+                    red_shared_if(&sc[opp(d)][ny][nx], f[d]);
+                }
+                atomicSub(&se[ly + 1][lx + 1], e_in - e);
             }
         }
-        __syncthreads_or(pushed);
+        if (threadIdx.x == 0) live[(s + 1) % 3] = 0;  // last read in sweep s - 2
+        __syncthreads();
         // relabel half: capacities and excess fixed
-        e = se[ly][lx];
-        if (e > 0 && hh < INF_H) {
+        e = se[ly + 1][lx + 1];
+        if (e > 0 && hh <= hlim) {
             int m = INF_H;
 #pragma unroll
-            for (int d = 0; d < ND; ++d)
-                if (sc[d][ly][lx] > 0) m = min(m, sh[ly + 1 + dyd(d)][lx + 1 + dxd(d)]);
+            for (int d = 0; d < ND; ++d) {
+                if (!on) hn[d] = sh[ly + 1 + dyd(d)][lx + 1 + dxd(d)];  // (others have them from the push half)
+                if (sc[d][ly + 1][lx + 1] > 0) m = min(m, hn[d]);
+            }
             if (m >= hh) {
                 hh = m >= INF_H - 1 ? INF_H : m + 1;
                 sh[ly + 1][lx + 1] = hh;
             }
         }
-        if (!__syncthreads_or(e > 0 && hh < INF_H)) break;
+        // still active?  A flag per sweep, three in rotation (set before a
+        // barrier, read after it, cleared two sweeps later)
+        if (__any_sync(0xffffffffu, e > 0 && hh <= hlim) && lx == 0) live[s % 3] = 1;
+        __syncthreads();
+        alive = live[s % 3] != 0;
+        if (!alive) break;
     }
+    if (alive && threadIdx.x == 0) g.due[t] = round + 1;
     if (inb) {
         g.h[i] = hh;
-        const int de = se[ly][lx] - e0;
+        const int de = se[ly + 1][lx + 1] - e0;
         if (de) atomicAdd(&g.e[i], de);
 #pragma unroll
         for (int d = 0; d < ND; ++d) {
-            const int dc = sc[d][ly][lx] - c0[d];
+            const int dc = sc[d][ly + 1][lx + 1] - c0[d];
             if (dc) atomicAdd(&g.cap[(long long)d * g.n + i], dc);
         }
     }
+    if (rx >= 0 && se[ry][rx]) {  // flow left the tile here (only toward pixels of the image: their heights are finite)
+        const int xx = x - lx + rx - 1, yy = y - ly + ry - 1;
+        const long long j = (long long)yy * g.W + xx;
+        atomicAdd(&g.e[j], se[ry][rx]);
+#pragma unroll
+        for (int d = 0; d < ND; ++d)
+            if (sc[d][ry][rx]) atomicAdd(&g.cap[(long long)d * g.n + j], sc[d][ry][rx]);
+        g.due[(yy / T8H) * tiles_x + xx / T8W] = round + 1;  // the tile it reached, in the next round
+    }
     __syncthreads();  // the shared arrays are reused by the block's next tile
-    return true;
 }
 
-// ---- exact global relabel: Bellman-Ford rounds over 32x32 tiles ----
+// ---- exact global relabel: a bit-parallel BFS per 32x32 tile ----
 // Heights are 1 on the sink-connected pixels (excess < 0) and otherwise
 // 1 + the fewest residual edges to one of them (INF when there is none), as a
-// frontier BFS from those pixels would give.  A round visits every tile once:
-// the tile's heights and a ring of its neighbours' heights go to shared
-// memory, h(u) = min(h(u), 1 + min over residual u -> v of h(v)) is swept to
-// the tile's fixpoint, and the heights go back.  Every height ever written is
-// the length of a real path to the sink (or INF), so a neighbour that reads a
-// height mid-round reads a valid upper bound; a round in which no tile
-// changed a height leaves every residual edge with h(u) <= h(v) + 1, which
-// with those upper bounds makes every height exact.  A shortest path about
-// as long as a tile side crosses few tiles, so a relabel takes a few rounds
-// (grid barriers) where a level-synchronous BFS takes one per level.
+// frontier BFS from those pixels would give.  First every tile's residual
+// edges, sinks and active pixels become row masks (mask8_tile); then rounds
+// over the tiles, one warp per tile with lane = row: a BFS of the whole tile
+// from its sinks and from its ring's heights, eight directions by shifts and
+// shuffles of the masks (bfs8_tile).  In round 0 the ring is the neighbours'
+// sinks; in a later round a tile whose ring would lower one of its border
+// pixels does its BFS again.  Every height ever written is the length of a
+// real path to the sink (or INF), so a neighbour that reads a height
+// mid-round reads a valid upper bound; a round in which no tile had a border
+// pixel to lower leaves every residual edge with h(u) <= h(v) + 1, which with
+// those upper bounds makes every height exact.  A shortest path about as long
+// as a tile side crosses few tiles, so a relabel takes a few rounds (grid
+// barriers) where a level-synchronous BFS takes one per level.
+//
+// (The relabel this replaced swept each tile to its fixpoint in shared memory,
+// reading 36 KB of capacities per tile and round.)  A round of a 640x480 graph
+// takes 8.4 us, of which the grid barrier is 2: the latency of one warp's BFS,
+// 40 to 60 levels.
 constexpr int G8W = 32, G8H = 32;
 constexpr int G8_ROWS = G8H / 8;  // rows per thread (256 threads)
+constexpr int NPLANE = 11;        // mask planes of a tile: 8 directions, excess < 0, excess > 0, reached by the BFS
+constexpr int PL_NEG = 8, PL_POS = 9, PL_REACH = 10;
+constexpr unsigned FULL8 = 0xffffffffu;
 
-// first: the stored heights are stale, so every height starts from the seed
-// (1 if excess < 0, else INF) and the ring reads seeds from the excess too.
-// Returns whether a height of the tile ended below its value at the start of
-// the visit (the value a neighbour may have read).
-__device__ bool gr8_tile(const G8 &g, int t, int tiles_x, bool first) {
-    __shared__ int gh[G8H + 2][G8W + 2];
-    const int lx = threadIdx.x & 31, wy = threadIdx.x >> 5;
-    const int x0 = (t % tiles_x) * G8W, y0 = (t / tiles_x) * G8H;
-    auto outside = [&](int xx, int yy) { return xx < 0 || yy < 0 || xx >= g.W || yy >= g.H; };
-    auto height = [&](long long j) -> int {
-        return first ? (g.e[j] < 0 ? 1 : INF_H) : *(volatile const int *)&g.h[j];
-    };
-    auto ring = [&](int xx, int yy) -> int {
-        return outside(xx, yy) ? INF_H : height((long long)yy * g.W + xx);
-    };
-    unsigned rm[G8_ROWS];  // residual directions of this thread's pixels (bit d: cap toward d > 0)
-    int h0[G8_ROWS];
+__device__ __forceinline__ const unsigned *plane8(const G8 &g, int t, int k) {
+    return g.tm + ((size_t)t * NPLANE + k) * 32;
+}
+
+// Mask planes of tile t (one block).
+__device__ void mask8_tile(const G8 &g, int t, int tiles_x) {
+    const int lane = threadIdx.x & 31, wy = threadIdx.x >> 5;
+    const int x = (t % tiles_x) * G8W + lane, y0 = (t / tiles_x) * G8H;
 #pragma unroll
     for (int k = 0; k < G8_ROWS; ++k) {
-        const int ly = wy + 8 * k, x = x0 + lx, y = y0 + ly;
-        int hv = INF_H;
-        unsigned m = 0;
-        if (!outside(x, y)) {
-            const long long i = (long long)y * g.W + x;
-            hv = height(i);
-            if (hv != 1) {
+        const int ly = wy + 8 * k, y = y0 + ly;
+        const bool in = x < g.W && y < g.H;
+        const long long i = (long long)y * g.W + x;
+        int c[ND];
 #pragma unroll
-                for (int d = 0; d < ND; ++d) m |= (g.cap[(long long)d * g.n + i] > 0 ? 1u : 0u) << d;
-            }
+        for (int d = 0; d < ND; ++d) c[d] = in ? __ldcg(g.cap + (long long)d * g.n + i) : 0;
+        const int e = in ? __ldcg(g.e + i) : 0;
+        unsigned w = 0;
+#pragma unroll
+        for (int d = 0; d < ND; ++d) {
+            const unsigned m = __ballot_sync(FULL8, c[d] > 0);
+            if (lane == d) w = m;
         }
-        rm[k] = m;
-        h0[k] = hv;
-        gh[ly + 1][lx + 1] = hv;
+        const unsigned neg = __ballot_sync(FULL8, e < 0), pos = __ballot_sync(FULL8, e > 0);
+        if (lane == PL_NEG) w = neg;
+        if (lane == PL_POS) w = pos;
+        if (lane <= PL_POS) g.tm[((size_t)t * NPLANE + lane) * 32 + ly] = w;
     }
-    if (wy == 0) gh[0][lx + 1] = ring(x0 + lx, y0 - 1);
-    if (wy == 1) gh[G8H + 1][lx + 1] = ring(x0 + lx, y0 + G8H);
-    if (wy == 2) gh[lx + 1][0] = ring(x0 - 1, y0 + lx);
-    if (wy == 3) gh[lx + 1][G8W + 1] = ring(x0 + G8W, y0 + lx);
-    if (wy == 4 && lx < 4) {
-        const int cx = lx & 1 ? G8W + 1 : 0, cy = lx & 2 ? G8H + 1 : 0;
-        gh[cy][cx] = ring(x0 - 1 + cx, y0 - 1 + cy);
-    }
-    __syncthreads();
-    // A tile's fixpoint takes at most one sweep per pixel of the tile (plus
-    // the sweep that sees no change); a visit that stops at the bound has
-    // changed heights, so another round follows.
-    for (int s = 0; s <= G8W * G8H; ++s) {
-        bool ch = false;
+}
+
+// Heights around a tile: hl / hr beside the lane's row, ht / hb above and
+// below column `lane`, and the four corners (the same in every lane).
+struct Ring8 {
+    int hl, hr, ht, hb, tl, tr, bl, br;
+};
+
+// Smallest ring level above lvl (warp-uniform), INF when there is none.
+__device__ __forceinline__ int next_ring8(const Ring8 &q, int lvl) {
+    int m = INF_H;
+    const int v[8] = {q.hl, q.hr, q.ht, q.hb, q.tl, q.tr, q.bl, q.br};
 #pragma unroll
-        for (int k = 0; k < G8_ROWS; ++k) {
-            if (!rm[k]) continue;
-            const int ly = wy + 8 * k;
-            int m = INF_H;
+    for (int k = 0; k < 8; ++k)
+        if (v[k] > lvl) m = min(m, v[k]);
+    return __reduce_min_sync(FULL8, m);
+}
+
+// Scratch of one warp: the index of the expansion that reached each pixel as
+// bit planes per row, and the level of each index.
+constexpr int B8_PL = 7, B8_IDX = 1 << B8_PL;
+struct Bfs8Scratch {
+    unsigned pl[B8_PL][32], reached[32], base[32];
+    int lv[B8_IDX];
+};
+
+// BFS of the tile with first pixel (x0, y0) on its planes m, the ring q; the
+// heights go to g.h.  A pixel's expansion index is kept in bit planes and the
+// heights are written row by row afterwards (coalesced); after B8_IDX
+// expansions the levels so far are written and the planes start again.
+__device__ unsigned bfs8_tile(const G8 &g, int x0, int y0, const unsigned m[9], const Ring8 &q, int hlim,
+                              Bfs8Scratch &sc) {
+    const int lane = threadIdx.x & 31;
+    unsigned S = m[PL_NEG], base = 0u, P[B8_PL];
 #pragma unroll
-            for (int d = 0; d < ND; ++d)
-                if ((rm[k] >> d) & 1u) m = min(m, gh[ly + 1 + dyd(d)][lx + 1 + dxd(d)]);
-            const int nh = m >= INF_H - 1 ? INF_H : m + 1;
-            if (nh < gh[ly + 1][lx + 1]) {
-                gh[ly + 1][lx + 1] = nh;
-                ch = true;
-            }
+    for (int k = 0; k < B8_PL; ++k) P[k] = 0u;
+    if (lane == 0) sc.lv[0] = 1;
+    int nidx = 4, lvl = 1;  // index 0: the seeds; expansions in fours from 4 on
+    auto expand = [&](unsigned S, int lvl) -> unsigned {
+        const unsigned T = __ballot_sync(FULL8, q.ht <= lvl), B = __ballot_sync(FULL8, q.hb <= lvl);
+        const unsigned side = (q.hl <= lvl ? 1u : 0u) | (q.hr <= lvl ? 0x80000000u : 0u);  // ring beside this row
+        unsigned up = __shfl_up_sync(FULL8, S, 1), dn = __shfl_down_sync(FULL8, S, 1);
+        unsigned su = __shfl_up_sync(FULL8, side, 1), sd = __shfl_down_sync(FULL8, side, 1);  // beside the rows above, below
+        if (lane == 0) {
+            up = T;
+            su = (q.tl <= lvl ? 1u : 0u) | (q.tr <= lvl ? 0x80000000u : 0u);
         }
-        if (!__syncthreads_or(ch)) break;
-    }
-    bool changed = false;
+        if (lane == 31) {
+            dn = B;
+            sd = (q.bl <= lvl ? 1u : 0u) | (q.br <= lvl ? 0x80000000u : 0u);
+        }
+        const unsigned near = (m[0] & ((S << 1) | (side & 1u))) | (m[1] & ((S >> 1) | (side & 0x80000000u))) |
+                              (m[2] & up) | (m[3] & dn);
+        const unsigned diag = (m[4] & ((up << 1) | (su & 1u))) | (m[5] & ((up >> 1) | (su & 0x80000000u))) |
+                              (m[6] & ((dn << 1) | (sd & 1u))) | (m[7] & ((dn >> 1) | (sd & 0x80000000u)));
+        return (near | diag) & ~S;
+    };
+    auto flush = [&](bool final) {
 #pragma unroll
-    for (int k = 0; k < G8_ROWS; ++k) {
-        const int ly = wy + 8 * k, x = x0 + lx, y = y0 + ly;
-        if (outside(x, y)) continue;
-        const int hv = gh[ly + 1][lx + 1];
-        if (first || hv != h0[k]) g.h[(long long)y * g.W + x] = hv;
-        changed |= hv != h0[k];
+        for (int k = 0; k < B8_PL; ++k) sc.pl[k][lane] = P[k];
+        sc.reached[lane] = S;
+        sc.base[lane] = base;
+        __syncwarp();
+        const unsigned bit = 1u << lane;
+        const bool col_in = x0 + lane < g.W;
+#pragma unroll 4
+        for (int r = 0; r < 32; ++r) {
+            const unsigned sr = sc.reached[r], br = sc.base[r];
+            int idx = 0;
+#pragma unroll
+            for (int k = 0; k < B8_PL; ++k) idx |= (int)((sc.pl[k][r] >> lane) & 1u) << k;
+            const bool fresh = ((sr & ~br) & bit) != 0;
+            const int v = fresh ? sc.lv[idx] : INF_H;
+            if (col_in && y0 + r < g.H && (fresh || (final && !(sr & bit))))
+                g.h[(long long)(y0 + r) * g.W + x0 + lane] = v;
+        }
+        __syncwarp();
+#pragma unroll
+        for (int k = 0; k < B8_PL; ++k) P[k] = 0u;
+        base = S;
+        nidx = 0;
+    };
+    // four levels per vote; a BFS ends after at most one expansion per pixel
+    // and ring level.  The four of a vote share the upper bits of their index.
+    for (int it = 0; it < G8W * G8H + 4 * 32 + 8 && lvl < hlim; ++it) {
+        const unsigned nw1 = expand(S, lvl);
+        const unsigned S1 = S | nw1;
+        const unsigned nw2 = expand(S1, lvl + 1);
+        const unsigned S2 = S1 | nw2;
+        const unsigned nw3 = expand(S2, lvl + 2);
+        const unsigned S3 = S2 | nw3;
+        const unsigned nw4 = expand(S3, lvl + 3);
+        const unsigned all = nw1 | nw2 | nw3 | nw4;
+        if (__any_sync(FULL8, all != 0)) {
+            if (nidx + 4 > B8_IDX) flush(false);
+            P[0] |= nw2 | nw4;
+            P[1] |= nw3 | nw4;
+#pragma unroll
+            for (int k = 2; k < B8_PL; ++k)
+                if ((nidx >> k) & 1) P[k] |= all;  // warp-uniform
+            if (lane < 4) sc.lv[nidx + lane] = lvl + 1 + lane;
+            S = S3 | nw4;
+            nidx += 4;
+            lvl += 4;
+        } else {
+            const int nxt = next_ring8(q, lvl + 3);
+            if (nxt >= INF_H) break;
+            lvl = nxt;
+        }
     }
-    return __syncthreads_or(changed);  // also: gh is reused by the block's next tile
+    flush(true);
+    return S;
+}
+
+// One warp's visit of tile t in a relabel round.  Returns whether it did the
+// BFS (round 0: always).
+__device__ bool gr8_tile(const G8 &g, int t, int tiles_x, int tiles_y, bool round0, int hlim,
+                         Bfs8Scratch &sc) {
+    const int lane = threadIdx.x & 31;
+    const int tx = t % tiles_x, ty = t / tiles_x;
+    const int x0 = tx * G8W, y0 = ty * G8H;
+    unsigned m[9];
+#pragma unroll
+    for (int k = 0; k < 9; ++k) m[k] = __ldcg(plane8(g, t, k) + lane);
+    Ring8 q;
+    if (round0) {
+        const bool L = tx > 0, R = tx < tiles_x - 1, U = ty > 0, D = ty < tiles_y - 1;
+        // sinks of the neighbour tile at offset o from t: row `row`, bit x
+        auto sink = [&](bool there, int o, int row, int x) {
+            return there && ((__ldcg(plane8(g, t + o, PL_NEG) + row) >> x) & 1u) ? 1 : INF_H;
+        };
+        q.hl = sink(L, -1, lane, 31);
+        q.hr = sink(R, 1, lane, 0);
+        q.ht = sink(U, -tiles_x, 31, lane);
+        q.hb = sink(D, tiles_x, 0, lane);
+        q.tl = sink(U && L, -tiles_x - 1, 31, 31);
+        q.tr = sink(U && R, -tiles_x + 1, 31, 0);
+        q.bl = sink(D && L, tiles_x - 1, 0, 31);
+        q.br = sink(D && R, tiles_x + 1, 0, 0);
+    } else {
+        auto at = [&](int xx, int yy) -> int {
+            return xx < 0 || yy < 0 || xx >= g.W || yy >= g.H ? INF_H : *(volatile const int *)&g.h[(long long)yy * g.W + xx];
+        };
+        q.hl = at(x0 - 1, y0 + lane);
+        q.hr = at(x0 + G8W, y0 + lane);
+        q.ht = at(x0 + lane, y0 - 1);
+        q.hb = at(x0 + lane, y0 + G8H);
+        q.tl = at(x0 - 1, y0 - 1);
+        q.tr = at(x0 + G8W, y0 - 1);
+        q.bl = at(x0 - 1, y0 + G8H);
+        q.br = at(x0 + G8W, y0 + G8H);
+        // would the ring lower a border pixel?  Each side: the least ring level
+        // that a border pixel's residual edges reach, against its own height.
+        const int ol = at(x0, y0 + lane), orr = at(x0 + G8W - 1, y0 + lane);
+        const int ot = at(x0 + lane, y0), ob = at(x0 + lane, y0 + G8H - 1);
+        auto edge = [](unsigned w, int x, int h) { return (w >> x) & 1u ? h : INF_H; };
+        // left and right columns (lane = row): straight, and the diagonals to the ring beside rows lane -+ 1
+        int lu = __shfl_up_sync(FULL8, q.hl, 1), ld = __shfl_down_sync(FULL8, q.hl, 1);
+        int ru = __shfl_up_sync(FULL8, q.hr, 1), rd = __shfl_down_sync(FULL8, q.hr, 1);
+        int tl = __shfl_up_sync(FULL8, q.ht, 1), tr = __shfl_down_sync(FULL8, q.ht, 1);
+        int bl = __shfl_up_sync(FULL8, q.hb, 1), br = __shfl_down_sync(FULL8, q.hb, 1);
+        if (lane == 0) { lu = q.tl; ru = q.tr; tl = q.tl; bl = q.bl; }
+        if (lane == 31) { ld = q.bl; rd = q.br; tr = q.tr; br = q.br; }
+        const int vl = min(edge(m[0], 0, q.hl), min(edge(m[4], 0, lu), edge(m[6], 0, ld)));
+        const int vr = min(edge(m[1], 31, q.hr), min(edge(m[5], 31, ru), edge(m[7], 31, rd)));
+        // top and bottom rows (lane = column): the masks of rows 0 and 31
+        const int vt = min(edge(__shfl_sync(FULL8, m[2], 0), lane, q.ht),
+                           min(edge(__shfl_sync(FULL8, m[4], 0), lane, tl), edge(__shfl_sync(FULL8, m[5], 0), lane, tr)));
+        const int vb = min(edge(__shfl_sync(FULL8, m[3], 31), lane, q.hb),
+                           min(edge(__shfl_sync(FULL8, m[6], 31), lane, bl), edge(__shfl_sync(FULL8, m[7], 31), lane, br)));
+        const bool imp = (vl < hlim && vl + 1 < ol) || (vr < hlim && vr + 1 < orr) || (vt < hlim && vt + 1 < ot) ||
+                         (vb < hlim && vb + 1 < ob);
+        if (!__any_sync(FULL8, imp)) return false;
+    }
+    g.tm[((size_t)t * NPLANE + PL_REACH) * 32 + lane] = bfs8_tile(g, x0, y0, m, q, hlim, sc);
+    return true;
 }
 
 // ---- the source-side closure (S_min) by rounds over 32x32 tiles ----
@@ -438,51 +618,80 @@ __global__ void __launch_bounds__(256) k8_solve(G8 g, P8 prm) {
     bool finished = false;
     int R = 0;  // tile and relabel rounds so far in this solve (grid-uniform)
     const int gtiles_x = (g.W + G8W - 1) / G8W;
-    const int gtiles = gtiles_x * ((g.H + G8H - 1) / G8H);
+    const int gtiles_y = (g.H + G8H - 1) / G8H, gtiles = gtiles_x * gtiles_y;
+    __shared__ Bfs8Scratch sc[8];
+    __shared__ unsigned s_todo;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int swarp = warp * gridDim.x + blockIdx.x, nwarps = gridDim.x * 8;  // block-interleaved warp rank
     for (int outer = 0; outer < prm.max_outer; ++outer) {
-        // ---- exact global relabel (gr8_tile rounds) ----
+        // ---- exact global relabel (mask8_tile, then gr8_tile rounds); with a
+        // height limit one further round after round 0, and heights that may
+        // come out too high ----
         // The round counters are the tile rounds' (round_active, R), with the
         // same clearing rule.
+        const int hlim = outer == 0 && prm.near_h > 0 ? prm.near_h : INF_H - 1;
+        if (gtid == 0) c->active = 0;
+        for (int t = blockIdx.x; t < gtiles; t += gridDim.x) mask8_tile(g, t, gtiles_x);
+        if (!sync8(c)) return;
         for (int q = 0;; ++q) {
-            if (gtid == 0) {
-                c->round_active[(R + 1) % 3] = 0;
-                if (q == 0) c->active = 0;
-            }
+            if (gtid == 0) c->round_active[(R + 1) % 3] = 0;
             int changed = 0;
-            for (int t = blockIdx.x; t < gtiles; t += gridDim.x) changed += gr8_tile(g, t, gtiles_x, q == 0);
-            if (threadIdx.x == 0 && changed) atomicAdd(&c->round_active[R % 3], changed);
+            for (int t = swarp; t < gtiles; t += nwarps)
+                changed += gr8_tile(g, t, gtiles_x, gtiles_y, q == 0, hlim, sc[warp]);
+            if (lane == 0 && changed) atomicAdd(&c->round_active[R % 3], changed);
             if (gtid == 0) c->gr_rounds++;
             if (!sync8(c)) return;
             const int more = *(volatile int *)&c->round_active[R % 3];
             ++R;
-            if (!more) break;
+            if (!more || (hlim < INF_H - 1 && q == 1)) break;
             if (q > g.n) {  // unreachable: a round makes at least one more path segment exact
                 if (gtid == 0) set_err8(c, E8_OUTER);
                 return;
             }
         }
         if (gtid == 0) c->global_relabels++;
-        // ---- count: excess that can still reach the sink ----
-        // one atomic per warp: per-thread atomics on one address serialise in L2
+        // ---- count: excess that can still reach the sink (lane = row of a
+        // 32x32 tile), and the tiles of the first round ----
         unsigned act = 0;
-        for (long long i = gtid; i < g.n; i += nth) act += g.e[i] > 0 && g.h[i] < INF_H;
+        const int tiles_x = (g.W + T8W - 1) / T8W, tiles_y = (g.H + T8H - 1) / T8H;
+        const int ntiles = tiles_x * tiles_y;
+        for (int t = swarp; t < gtiles; t += nwarps) {
+            const unsigned w = __ldcg(plane8(g, t, PL_POS) + lane) & __ldcg(plane8(g, t, PL_REACH) + lane);
+            act += __popc(w);
+            const unsigned rows = __ballot_sync(FULL8, w != 0);
+            const int ty8 = (t / gtiles_x) * (G8H / T8H) + lane;  // lanes 0..3: the tile's 32x8 quarters
+            if (lane < G8H / T8H && ((rows >> (T8H * lane)) & 0xFFu)) g.due[ty8 * tiles_x + t % gtiles_x] = R;
+        }
         act = __reduce_add_sync(0xffffffffu, act);
         if ((threadIdx.x & 31) == 0 && act) atomicAdd(&c->active, (unsigned long long)act);
+        if (gtid == 0) c->round_active[(R + 1) % 3] = 0;
         if (!sync8(c)) return;
         if (*(volatile unsigned long long *)&c->active == 0) {
+            if (hlim < INF_H - 1) continue;  // none within the limit: the exact relabel next
             finished = true;
             break;
         }
-        // ---- tile rounds: every tile once per round, block-local sweeps ----
-        const int tiles_x = (g.W + T8W - 1) / T8W;
-        const int ntiles = tiles_x * ((g.H + T8H - 1) / T8H);
+        // ---- tile rounds: the due tiles, block-local sweeps ----
         for (int p = 0; p < prm.rounds; ++p) {
-            // round_active[R % 3] counts this round's tiles with work and is read
-            // after the round's barrier; the counter of round R + 1 was last read
-            // after the barrier of round R - 2, which every block has passed
+            // round_active[R % 3] counts this round's tiles and is read after the
+            // round's barrier; the counter of round R + 1 was last read after
+            // the barrier of round R - 2, which every block has passed
             if (gtid == 0) c->round_active[(R + 1) % 3] = 0;
             int worked = 0;
-            for (int t = blockIdx.x; t < ntiles; t += gridDim.x) worked += tile8_visit(g, t, tiles_x, prm.sweeps);
+            // the block's tiles 32 at a time, their stamps in one load
+            for (int tb = blockIdx.x; tb < ntiles; tb += 32 * gridDim.x) {  // block-uniform
+                const int mine = tb + lane * gridDim.x;
+                unsigned todo = __ballot_sync(FULL8, mine < ntiles && *(volatile int *)(g.due + mine) >= R);
+                // (a neighbour may raise a stamp meanwhile: thread 0's reading decides for the block)
+                if (threadIdx.x == 0) s_todo = todo;
+                __syncthreads();
+                todo = s_todo;
+                for (; todo; todo &= todo - 1) {
+                    tile8_visit(g, tb + (__ffs(todo) - 1) * gridDim.x, tiles_x, prm.sweeps, hlim, R);
+                    ++worked;
+                }
+                __syncthreads();
+            }
             if (threadIdx.x == 0 && worked) {
                 atomicAdd(&c->round_active[R % 3], worked);
                 atomicAdd(&c->tile_visits, (unsigned long long)worked);
@@ -556,14 +765,18 @@ struct gcfg_graph8 {
     int32_t penalty = 0;
     bool varying = false, built = false, solved = false;
     int *cap = nullptr, *e = nullptr, *h = nullptr, *mark = nullptr;
+    unsigned *tm = nullptr;
+    int *due = nullptr;
     int32_t *d_label = nullptr;
     Ctl8 *ctl = nullptr, *h_ctl = nullptr;
     cudaStream_t st = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev2 = nullptr;  // solve start, solve end, extract end
-    // schedule (measured on a 640x480 graph with a constant penalty of 600,
-    // 8 sweeps per visit, solve kernel time: 12 tile rounds per global
-    // relabel take 0.96 ms at 3 blocks per SM and 1.03 ms at 2; 8 rounds
-    // 0.99 ms, 16 rounds 1.05 ms, 32 rounds 1.17 ms, 4 rounds 1.20 ms)
+    // schedule: 8 sweeps per visit; solve kernel at 12 / 8 / 6 / 4 tile rounds
+    // per global relabel: 640x480, penalty 600 957 / 963 / 978 / 1040 us, penalty
+    // 20 497 / 385 / 348 / 503, arrays 351 / 272 / 231 / 194, 1920x1080 penalty 600
+    // 3285 / 3344 / 3734 / 4182 (16 sweeps: 1102 / 991 / 980 / 1024, 579 / 471 /
+    // 428 / 397, 499 / 372 / 309 / 245, 3486 / 3517 / 3599 / 4039); 2 blocks per
+    // SM are as fast as 3
     int rounds = GCFG_N8_ROUNDS, max_outer = 100000, blocks_per_sm = 3, sweeps = GCFG_N8_SWEEPS;
 
     G8 g() const {
@@ -575,12 +788,14 @@ struct gcfg_graph8 {
         x.e = e;
         x.h = h;
         x.mark = mark;
+        x.tm = tm;
+        x.due = due;
         x.ctl = ctl;
         return x;
     }
     void release() {
         cudaFree(cap); cudaFree(e); cudaFree(h); cudaFree(mark);
-        cudaFree(d_label); cudaFree(ctl);
+        cudaFree(d_label); cudaFree(ctl); cudaFree(tm); cudaFree(due);
         if (h_ctl) cudaFreeHost(h_ctl);
         if (ev0) cudaEventDestroy(ev0);
         if (ev1) cudaEventDestroy(ev1);
@@ -634,6 +849,7 @@ gcfg_status gcfg_set_stream8(gcfg_graph8 *g, void *stream) {
 gcfg_status gcfg_set_graph8(gcfg_graph8 *g) {
     if (!g || !g->dp || !g->dn) return GCFG_ERR_STATE;
     GCFG_CK(cudaMemsetAsync(g->ctl, 0, sizeof(Ctl8), g->st));
+    GCFG_CK(cudaMemsetAsync(g->due, 0xff, (size_t)((g->W + 31) / 32) * ((g->H + 7) / 8) * sizeof(int), g->st));
     Arr8 arr;
     for (int d = 0; d < 8; ++d) arr.a[d] = g->varying ? g->arr[d] : nullptr;
     k8_build<<<grid8(g->n), 256, 0, g->st>>>(g->g(), g->dp, g->dn, g->penalty, arr);
@@ -662,7 +878,9 @@ gcfg_status gcfg_init8(int w, int h, const int32_t *dp, const int32_t *dn, int32
     gcfg_status rc = GCFG_OK;
     if (cudaMalloc(&g->cap, 8 * n * sizeof(int)) != cudaSuccess || cudaMalloc(&g->e, n * sizeof(int)) != cudaSuccess ||
         cudaMalloc(&g->h, n * sizeof(int)) != cudaSuccess || cudaMalloc(&g->mark, n * sizeof(int)) != cudaSuccess ||
-        cudaMalloc(&g->d_label, n * sizeof(int)) != cudaSuccess || cudaMalloc(&g->ctl, sizeof(Ctl8)) != cudaSuccess ||
+        cudaMalloc(&g->d_label, n * sizeof(int)) != cudaSuccess ||
+        cudaMalloc(&g->tm, (size_t)((w + 31) / 32) * ((h + 31) / 32) * NPLANE * 32 * sizeof(unsigned)) != cudaSuccess ||
+        cudaMalloc(&g->due, (size_t)((w + 31) / 32) * ((h + 7) / 8) * sizeof(int)) != cudaSuccess || cudaMalloc(&g->ctl, sizeof(Ctl8)) != cudaSuccess ||
         cudaMallocHost(&g->h_ctl, sizeof(Ctl8)) != cudaSuccess)
         rc = GCFG_ERR_OOM;
     if (rc == GCFG_OK && (cudaEventCreate(&g->ev0) != cudaSuccess || cudaEventCreate(&g->ev1) != cudaSuccess ||
@@ -694,7 +912,12 @@ gcfg_status gcfg_optimize8(gcfg_graph8 *g, int32_t *host_label, gcfg_result *res
     long long grid = (long long)(per_sm > 0 ? per_sm : 1) * (sms > 0 ? sms : 1);
     if (want < grid) grid = want > 0 ? want : 1;
     G8 gg = g->g();
-    P8 prm{g->max_outer, g->rounds, g->sweeps};
+    // A height limit for the first iteration pays where edges saturate, as
+    // contrast-sensitive ones do; a constant penalty leaves most of them
+    // open, flow has to travel, and the limited iteration is in the way
+    // (640x480 / 1920x1080, us without -> with: arrays 272 -> 177, 602 -> 393;
+    // penalty 600 963 -> 995, 3344 -> 4285).
+    P8 prm{g->max_outer, g->rounds, g->sweeps, g->varying ? 9 : 0};
     void *args[] = {&gg, &prm};
     GCFG_CK(cudaEventRecord(g->ev0, g->st));
     GCFG_CK(cudaLaunchCooperativeKernel((const void *)k8_solve, dim3((unsigned)grid), dim3(256), args, 0, g->st));
