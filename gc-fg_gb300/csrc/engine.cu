@@ -520,7 +520,7 @@ struct SmemPush {
     int nrec;
     unsigned dirty, dirty_h;  // rows whose capacities or excess, and whose heights, changed
     unsigned long long part[NW];
-    int idx;
+    int idx;  // the block's next queue entry
 };
 template <int NW>
 struct SmemWarp {  // one of each per warp: the global relabel's tile BFS
@@ -778,9 +778,77 @@ __device__ void sink_reach_tile(const Batch &b, int t, bool round0, int tag_next
 // Push/relabel on one tile (whole block)
 // ---------------------------------------------------------------------------
 
-// The block's next queue entry is taken (from take_ctr) when the sweeps end,
-// so that the atomic overlaps the write-back; it is left in s.idx for the
-// caller.
+// A block's way through a phase's queue of n tiles: block i starts with entry
+// i, the entries past the grid's size are taken one by one from a counter.
+struct Queue {
+    const int *list;
+    int *take;
+    int n;
+    int idx, t;  // this visit's entry and tile (-1: no more)
+    __device__ __forceinline__ void open(const int *l, int *tk, int size) {
+        list = l;
+        take = tk;
+        n = size;
+        move((int)blockIdx.x);
+    }
+    __device__ __forceinline__ void move(int i) {
+        idx = i;
+        t = i < n ? __ldcg(list + i) : -1;
+    }
+};
+
+// A visit's hand-over of the flow into its halo, one lane per border pixel of
+// warps 0..3 (left, right, upper, lower neighbour tile nt, or -1): begin adds
+// the flow to the pixel across the border, finish uses what the adds returned.
+// Every visit's hand-over is finished by the block's next visit of the same
+// phase, or at the latest before the phase's barrier.
+template <int NW>
+struct HandOver {
+    int nt = -1, f = 0, old_e = 0, old_c = 0;
+    int own = -1;  // the visited tile, if it is still active: due in its colour's next phase
+    // left tile, its RIGHT edge; right tile, its LEFT edge; upper tile, its
+    // DOWN edge; lower tile, its UP edge
+    __device__ __forceinline__ static int warp() { return threadIdx.x >> 5; }
+    __device__ __forceinline__ static int px() {
+        const int lane = threadIdx.x & 31, w = warp();
+        return w == 0 ? lane * 32 + 31 : w == 1 ? lane * 32 : w == 2 ? 31 * 32 + lane : lane;
+    }
+    __device__ __forceinline__ void begin(const Batch &b, int flow) {
+        f = nt >= 0 ? flow : 0;
+        if (f) {
+            const size_t q = (size_t)nt * TPX + px();
+            old_e = atomicAdd(b.exc + q, f);
+            old_c = atomicAdd(reinterpret_cast<int *>(b.cap + q) + (warp() ^ 1), f);
+        }
+    }
+    __device__ __forceinline__ void finish(const Batch &b, int phase) {
+        if (threadIdx.x == (NW >= 8 ? 4 * 32 : 0) && own >= 0)
+            enqueue(b, b.mark_push, (phase + 2) % 3, phase + 2, own);
+        own = -1;
+        if (threadIdx.x >= 4 * 32) return;
+        bool activated = false;  // a pixel of nt now has excess: nt needs a visit
+        if (f) {
+            // keep the receiving tile's mask planes and excess sum exact
+            const int new_e = old_e + f;
+            unsigned *mt = b.tmask + (size_t)nt * 6 * 32;
+            const int row = px() >> 5;
+            const unsigned bit = 1u << (px() & 31);
+            if (old_c == 0) atomicOr(mt + (warp() ^ 1) * 32 + row, bit);
+            if (old_e < 0 && new_e >= 0) atomicAnd(mt + 4 * 32 + row, ~bit);
+            if (old_e <= 0 && new_e > 0) atomicOr(mt + 5 * 32 + row, bit);
+            const int dpos = max(new_e, 0) - max(old_e, 0);
+            if (dpos) atomicAdd(b.tile_pos + nt, (unsigned long long)dpos);
+            // flow that only fills sink capacity (the excess stays <= 0) leaves
+            // nothing to push there
+            activated = new_e > 0;
+        }
+        if (__any_sync(FULL, activated) && (threadIdx.x & 31) == 0)
+            enqueue(b, b.mark_push, (phase + 1) % 3, phase + 1, nt);
+        f = 0;
+    }
+};
+
+// Visits tile q.t and moves q to the block's next entry.
 //
 // What bounds a visit: a solve waits for its longest visits (at the end of a
 // phase most blocks are idle), so it is the latency of a sweep, and in a
@@ -788,44 +856,75 @@ __device__ void sink_reach_tile(const Batch &b, int t, bool round0, int tag_next
 // whether there is flow, and whether it stays in the tile, cost more than the
 // adds: with a ring around every array and 13 adds that never ask, a sweep
 // of one block alone takes, in cycles (half the pixels active / 3% active),
-// 16 warps 2426 -> 1596 / 1994 -> 1432, 8 warps 3611 -> 1873 (half active).
-// Only rows that changed are written back, and the next visit's loads start
-// without a barrier behind the hand-over.  Device time of a solve, before ->
-// with the adds -> with the write-back: 1920x1080 212 -> 204 -> 202 us,
-// 4096x4096 1069 -> 1012 -> 990, 256 uneven images 1530 -> 1493 -> 1424.
+// 16 warps 2426 -> 1645 / 1994 -> 1493, 8 warps 3611 -> 2057 (half active).
+// Only rows that changed are written back, the next visit's loads start
+// without a barrier behind the hand-over, and the dependent round trips to
+// memory (the queue's counter, the hand-over's results, the own tile's queue
+// entry) run beside the loads and sweeps.  Device time of a solve, before ->
+// with the adds -> with the write-back -> with the round trips: 1920x1080
+// 212 -> 204 -> 202 -> 200 us, 4096x4096 1069 -> 1012 -> 990 -> 990, 40 uneven
+// images 337 -> 325 -> 321 -> 314, 256 of them 1530 -> 1493 -> 1424 -> 1400.
+// Fetching the next tile into the L2 cache as well, or dealing the tiles out
+// in turn so that it is known earlier, gave no more (256 images 1385 to 1400
+// us, 4096x4096 997 to 1020): with four blocks per SM a large solve's visits
+// are bound by the instructions they issue.
 template <int NW>
-__device__ void push_tile(const Batch &b, int t, const SolveParams &prm, int hlim, int phase, SmemPush<NW> &s,
-                          unsigned long long *st, int *take_ctr) {
+__device__ __forceinline__ void push_tile(const Batch &b, Queue &q, const SolveParams &prm, int hlim, int phase,
+                                          SmemPush<NW> &s, HandOver<NW> &ho, unsigned long long *st) {
     constexpr int RPW = TILE_H / NW;  // rows per warp: thread (warp, lane) owns rows warp + NW k, column lane
+    constexpr int SVC = NW >= 8 ? 5 * 32 : 0;  // takes the queue entries: a warp without hand-over duty if there is one
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     // section times: 32-bit cycle counters (a visit is far shorter than 2^32 cycles)
     const unsigned c0 = (unsigned)clock();
     unsigned cb = 0;
-    GrGeo g;  // only the neighbours are used
-    tile_nbs(b, t, g.nb);
+    const int t = q.t;
+    // The next entry is taken now, so that the atomic's round trip is over when
+    // the visit ends, or, with fewer than two rounds of the grid left, when the
+    // visit ends, so that a block in a long visit holds nothing back.
+    const int grid = (int)gridDim.x;
+    const bool early = q.idx + 2 * grid < q.n;
+    int taken = q.n;
     const size_t base = (size_t)t * TPX;
+    {
+        int4 c[RPW];
+        int e[RPW], h[RPW];
 #pragma unroll
-    for (int k = 0; k < RPW; ++k) {
-        const int r = warp + NW * k;
-        const int4 c = __ldcg(b.cap + base + r * 32 + lane);
-        s.c[0][r + 1][lane + 1] = c.x;
-        s.c[1][r + 1][lane + 1] = c.y;
-        s.c[2][r + 1][lane + 1] = c.z;
-        s.c[3][r + 1][lane + 1] = c.w;
-        s.e[r + 1][lane + 1] = __ldcg(b.exc + base + r * 32 + lane);
-        s.h[r + 1][lane + 1] = __ldcg(b.h + base + r * 32 + lane);
+        for (int k = 0; k < RPW; ++k) {
+            const int r = warp + NW * k;
+            c[k] = __ldcg(b.cap + base + r * 32 + lane);
+            e[k] = __ldcg(b.exc + base + r * 32 + lane);
+            h[k] = __ldcg(b.h + base + r * 32 + lane);
+        }
+        if (threadIdx.x == SVC && early) taken = atomicAdd(q.take, 1);
+        ho.finish(b, phase);
+        int nb = -1;
+        if (warp < 4) {
+            // warps 0..3 each serve one side: left, right, upper, lower neighbour tile
+            int a[4];
+            tile_nbs(b, t, a);
+            nb = warp == 0 ? a[0] : warp == 1 ? a[1] : warp == 2 ? a[2] : a[3];
+            const int far = warp == 0 ? HB_RGT : warp == 1 ? HB_LFT : warp == 2 ? HB_BOT : HB_TOP;
+            const int v = nb >= 0 ? __ldcg(b.hb + (size_t)nb * 128 + far + lane) : INF_H;
+            const int y = warp == 2 ? 0 : warp == 3 ? TILE_H + 1 : lane + 1;
+            const int x = warp == 0 ? 0 : warp == 1 ? TILE_W + 1 : lane + 1;
+            s.h[y][x] = v;
+            // the ring of e collects the flow into the halo (that of c only takes
+            // the "capacity back" of such flow, which nothing reads); each cell is
+            // cleared by the lane that handed its last contents over
+            s.e[y][x] = 0;
+        }
+        ho.nt = nb;
+#pragma unroll
+        for (int k = 0; k < RPW; ++k) {
+            const int r = warp + NW * k;
+            s.c[0][r + 1][lane + 1] = c[k].x;
+            s.c[1][r + 1][lane + 1] = c[k].y;
+            s.c[2][r + 1][lane + 1] = c[k].z;
+            s.c[3][r + 1][lane + 1] = c[k].w;
+            s.e[r + 1][lane + 1] = e[k];
+            s.h[r + 1][lane + 1] = h[k];
+        }
     }
-    if (warp == 0) s.h[0][lane + 1] = g.nb[2] >= 0 ? __ldcg(b.hb + (size_t)g.nb[2] * 128 + HB_BOT + lane) : INF_H;
-    if (warp == 1) s.h[TILE_H + 1][lane + 1] = g.nb[3] >= 0 ? __ldcg(b.hb + (size_t)g.nb[3] * 128 + HB_TOP + lane) : INF_H;
-    if (warp == 2) s.h[lane + 1][0] = g.nb[0] >= 0 ? __ldcg(b.hb + (size_t)g.nb[0] * 128 + HB_RGT + lane) : INF_H;
-    if (warp == 3) s.h[lane + 1][TILE_W + 1] = g.nb[1] >= 0 ? __ldcg(b.hb + (size_t)g.nb[1] * 128 + HB_LFT + lane) : INF_H;
-    // the ring of e collects the flow into the halo (that of c only takes the
-    // "capacity back" of such flow, which nothing reads)
-    // Each cell is cleared by the lane that handed its last contents over.
-    if (warp == 0) s.e[lane + 1][0] = 0;
-    if (warp == 1) s.e[lane + 1][TILE_W + 1] = 0;
-    if (warp == 2) s.e[0][lane + 1] = 0;
-    if (warp == 3) s.e[TILE_H + 1][lane + 1] = 0;
     __syncthreads();
     const unsigned c1 = (unsigned)clock();
     if (threadIdx.x == 0) s.dirty = s.dirty_h = 0;  // every warp has read the last visit's
@@ -939,7 +1038,7 @@ __device__ void push_tile(const Batch &b, int t, const SolveParams &prm, int hli
                 atomicAdd(pe + PW, fd);
                 atomicAdd(pe, e - ev[k]);
                 pushed |= e != ev[k];
-                if (e != ev[k]) rows |= (1u << r) | (fu ? (1u << r) >> 1 : 0u) | (fd ? (1u << r) << 1 : 0u);
+                rows |= 1u << r | (fu ? (1u << r) >> 1 : 0u) | (fd ? (1u << r) << 1 : 0u);
             }
         }
         // block-uniform "anything pushed in this sweep" (every warp takes the
@@ -1000,32 +1099,24 @@ __device__ void push_tile(const Batch &b, int t, const SolveParams &prm, int hli
     }
     const unsigned c2 = (unsigned)clock();
     // Warps 0..3 hand the halo flow to the (idle) neighbour tiles: the adds
-    // first, so that their round trips overlap the write-back.
-    const int nt = warp == 0 ? g.nb[0] : warp == 1 ? g.nb[1] : warp == 2 ? g.nb[2] : warp == 3 ? g.nb[3] : -1;
-    int f = 0, old_e = 0, old_c = 0, line = 0;
-    // left tile, its RIGHT edge; right tile, its LEFT edge; upper tile, its
-    // DOWN edge; lower tile, its UP edge
-    const int px = warp == 0 ? lane * 32 + 31 : warp == 1 ? lane * 32 : warp == 2 ? 31 * 32 + lane : lane;
-    const int comp = warp ^ 1;
+    // here, so that their round trips overlap the write-back; what depends on
+    // their results when the next visit's loads are on their way.
+    int line = 0;
     if (warp < 4) {
-        f = warp == 0 ? s.e[lane + 1][0] : warp == 1 ? s.e[lane + 1][TILE_W + 1]
-          : warp == 2 ? s.e[0][lane + 1] : s.e[TILE_H + 1][lane + 1];
-        if (nt < 0) f = 0;
-        if (f) {
-            const size_t q = (size_t)nt * TPX + px;
-            old_e = atomicAdd(b.exc + q, f);
-            old_c = atomicAdd(reinterpret_cast<int *>(b.cap + q) + comp, f);
-        }
+        const int y = warp == 2 ? 0 : warp == 3 ? TILE_H + 1 : lane + 1;
+        const int x = warp == 0 ? 0 : warp == 1 ? TILE_W + 1 : lane + 1;
+        ho.begin(b, s.e[y][x]);
         // the border lines, for the neighbours' halos: HB_TOP, HB_BOT, HB_LFT, HB_RGT
         line = warp == 0 ? s.h[1][lane + 1] : warp == 1 ? s.h[TILE_H][lane + 1]
              : warp == 2 ? s.h[lane + 1][1] : s.h[lane + 1][TILE_W];
     }
-    // With 8 or more warps, warps without hand-over duty take the block's next
-    // queue entry and queue a tile still active for its colour's next phase
-    // (two dependent atomics; the slot of phase + 2 was emptied at the last
-    // barrier and is not read in this phase).
-    if (threadIdx.x == (NW >= 8 ? 5 * 32 : 0)) s.idx = atomicAdd(take_ctr, 1);
-    if (any && threadIdx.x == (NW >= 8 ? 4 * 32 : 0)) enqueue(b, b.mark_push, (phase + 2) % 3, phase + 2, t);
+    if (threadIdx.x == SVC) {
+        if (!early && q.n > grid) taken = atomicAdd(q.take, 1);
+        s.idx = grid + taken;
+    }
+    // a tile still active is queued for its colour's next phase (the slot of
+    // phase + 2 was emptied at the last barrier and is not read in this phase)
+    ho.own = any ? t : -1;
     // which rows changed, and the tile's sum of positive excess
     rows = __reduce_or_sync(FULL, rows);
     hrows = __reduce_or_sync(FULL, hrows);
@@ -1069,26 +1160,7 @@ __device__ void push_tile(const Batch &b, int t, const SolveParams &prm, int hli
         for (int w = 0; w < NW; ++w) tot += s.part[w];
         b.tile_pos[t] = tot;
     }
-    if (warp < 4) {
-        bool activated = false;  // a pixel of nt now has excess: nt needs a visit
-        if (f) {
-            // keep the receiving tile's mask planes and excess sum exact
-            const int new_e = old_e + f;
-            unsigned *mt = b.tmask + (size_t)nt * 6 * 32;
-            const int row = px >> 5;
-            const unsigned bit = 1u << (px & 31);
-            if (old_c == 0) atomicOr(mt + comp * 32 + row, bit);
-            if (old_e < 0 && new_e >= 0) atomicAnd(mt + 4 * 32 + row, ~bit);
-            if (old_e <= 0 && new_e > 0) atomicOr(mt + 5 * 32 + row, bit);
-            const int dpos = max(new_e, 0) - max(old_e, 0);
-            if (dpos) atomicAdd(b.tile_pos + nt, (unsigned long long)dpos);
-            // flow that only fills sink capacity (the excess stays <= 0) leaves
-            // nothing to push there
-            activated = new_e > 0;
-        }
-        if (__any_sync(FULL, activated) && lane == 0)
-            enqueue(b, b.mark_push, (phase + 1) % 3, phase + 1, nt);
-    }
+    q.move(s.idx);
     if (threadIdx.x == 0) {
         stat_add(st, ST_PUSH_TILES, 1ull);
         stat_add(st, ST_PUSH_SWEEPS, (unsigned long long)sweeps);
@@ -1433,20 +1505,13 @@ __global__ void __launch_bounds__(NW * 32, solve_min_blocks<NW>()) k_solve(Batch
                 const int slot = p % 3;
                 last = p;
                 const int n = vload(&ctl->size[slot]);
-                {
-                    const long long ct = clock64();
-                    if (threadIdx.x == 0) sm.p.idx = atomicAdd(&ctl->take[slot], 1);
-                    __syncthreads();
-                    if (threadIdx.x == 0) stat_add(st, ST_CYC_TAKE, (unsigned long long)(clock64() - ct));
-                }
-                for (;;) {
-                    // the entry taken before (the first one above, later ones by
-                    // the previous visit); no thread writes s.idx again before
-                    // every thread has read it (push_tile's barriers come first)
-                    const int idx = sm.p.idx;
-                    if (idx >= n) break;
-                    push_tile(b, b.lists[(size_t)slot * b.list_cap + idx], prm, hlim, p, sm.p, st, &ctl->take[slot]);
-                }
+                Queue q;
+                const long long ct = clock64();
+                q.open(b.lists + (size_t)slot * b.list_cap, &ctl->take[slot], n);
+                if (threadIdx.x == 0 && q.t >= 0) stat_add(st, ST_CYC_TAKE, (unsigned long long)(clock64() - ct));
+                HandOver<NW> ho;
+                while (q.t >= 0) push_tile(b, q, prm, hlim, p, sm.p, ho, st);
+                ho.finish(b, p);
                 // the phase's tail: from the first block out of work to the barrier
                 if (threadIdx.x == 0) atomicMax(&ctl->push_idle[p & 1], ~gtimer());
                 if (gtid == 0) ctl->push_idle[(p + 1) & 1] = 0;  // last read after the previous phase
