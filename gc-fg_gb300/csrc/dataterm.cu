@@ -160,16 +160,19 @@ __device__ __forceinline__ float ex2_approx(float z) {
     return r;
 }
 
+// The float fast path where q.small holds (see nlink_fast).
+__device__ __forceinline__ bool nlink_fast_small(int d2, const NlinkParams &q, int &w) {
+    const float v = q.lf * ex2_approx(-small_int_to_float(d2) * q.scale);
+    const float t = __fadd_rn(v, 12582912.0f);  // 1.5 * 2^23 + rint(v)
+    w = __float_as_int(t) - 0x4B400000;
+    return fabsf(__fsub_rn(v, __fsub_rn(t, 12582912.0f))) < q.half_margin;
+}
+
 // The float fast path: w = the rounded weight, true when v is farther than
 // the margin from a rounding boundary (else the double expression decides).
 __device__ __forceinline__ bool nlink_fast(int d2, const NlinkParams &q, int &w) {
+    if (q.small) return nlink_fast_small(d2, q, w);
     const float v = q.lf * ex2_approx(-small_int_to_float(d2) * q.scale);
-    if (q.small) {
-        const float t = __fadd_rn(v, 12582912.0f);  // 1.5 * 2^23 + rint(v)
-        const float rf = __fsub_rn(t, 12582912.0f);
-        w = __float_as_int(t) - 0x4B400000;
-        return fabsf(__fsub_rn(v, rf)) < q.half_margin;
-    }
     const float fr = v - floorf(v);
     w = (int)floorf(v + 0.5f);
     return fabsf(fr - 0.5f) > q.margin;
@@ -423,7 +426,7 @@ __global__ void __launch_bounds__(256, 8) k_hist_sigma_b(const uint8_t *__restri
 // image's n-link constants by the block's last thread.
 __global__ void __launch_bounds__(1024) k_tlut_b(const int *__restrict__ ilist, const int *__restrict__ hist,
                                                  const ImgDesc *__restrict__ img, ImgState *ist,
-                                                 int *__restrict__ dp_lut, int *__restrict__ dn_lut,
+                                                 int2 *__restrict__ tl_lut,
                                                  double *raw_dp, double *raw_dn) {
     __shared__ long long part[2][32];
     const int im = ilist ? ilist[blockIdx.x] : blockIdx.x;
@@ -472,8 +475,7 @@ __global__ void __launch_bounds__(1024) k_tlut_b(const int *__restrict__ ilist, 
             qdp = tlink_quant(hb[b], Nb);
             qdn = tlink_quant(hf[b], Nf);
         }
-        dp_lut[(size_t)im * NBINS + b] = qdp;
-        dn_lut[(size_t)im * NBINS + b] = qdn;
+        tl_lut[(size_t)im * NBINS + b] = make_int2(qdp, qdn);
     }
 }
 
@@ -486,274 +488,240 @@ __device__ __forceinline__ int nlink_w(int d2, const NlinkParams &q) {
 // Fused image -> residual graph of one tile: t-link gather, n-links, the
 // reference's interior/border conventions, tile-major output.
 //
-// The tile's colours and a 1-pixel halo are staged in shared memory as packed
-// words; every undirected edge between two interior pixels is weighed once
-// (the weight is symmetric in its two pixels) into a right-edge and a
-// down-edge table, and each pixel then reads its four capacities from them.
-// An edge that touches the 1-pixel image border has capacity 0, as in the
-// reference's graph (GraphCutKernels.cu:112-214).  Eight blocks per SM
-// (32 registers, a few spilled): more tiles in flight hide the staging loads
-// (batch256 0.426 ms at five blocks, 0.408 at six, 0.399 at eight).
-__global__ void __launch_bounds__(TILE_THREADS, 8) k_build_img_b(Batch b, const uint8_t *__restrict__ rgb,
-                                                               const int *__restrict__ dp_lut,
-                                                               const int *__restrict__ dn_lut) {
-    constexpr int SW = TILE_W + 2, SH = TILE_H + 2;
-    __shared__ uint32_t col[SH][SW];              // pixel (x0 - 1 + j, y0 - 1 + i)
-    __shared__ int wr[TILE_H][TILE_W + 1];        // edge (x, y)-(x + 1, y), x = x0 - 1 + j, y = y0 + i
-    __shared__ int wd[TILE_H + 1][TILE_W];        // edge (x, y)-(x, y + 1), x = x0 + j, y = y0 - 1 + i
+// A warp walks down a strip of rows, lane = column, and needs no other warp's
+// results: each lane reads its pixel and the one to the right as aligned words
+// (every line of the image's rows comes from L1 after the first of them), keeps
+// the row below's colour for the next row, and weighs the edges to the right
+// and down; the weight from the left comes from the next lane, that from above
+// from the row before.  A strip reads one row above and one below it again and
+// weighs the edges over its upper border a second time (the weight is symmetric
+// in its two pixels).  An edge that touches the 1-pixel image border has
+// capacity 0, as in the reference's graph (GraphCutKernels.cu:112-214).
+//
+// What bounds it: the instructions issued and, beside them, the shared-memory
+// and L1 pipe (a gather of random bins is up to 32 lines).  Staging the tile's
+// colours, then weighing all edges, then joining them, with a barrier between,
+// took 8300 warp instructions per tile; inside the image a strip needs none of
+// the border's checks and, with one 8-byte gather for both t-links, about
+// 4000.  256 uneven images (54,000 tiles) 420 -> 330 us, 4096x4096 135 -> 96
+// (400 MB at 4.2 TB/s), 1920x1080 23.6 -> 19.1.
+struct BuildTile {
+    int W, H, x, ys;        // image size, the lane's column, the strip's first row
+    const uint8_t *base;    // the image's first byte
+    const int2 *lut;
+    int4 *cap;              // the strip's first row in the arena, this lane's column
+    int *exc;
+    uint32_t (*msk)[TILE_H];
+    int r0;                 // the strip's first row within the tile
+};
+
+// What a tile needs.  INNER: the tile and the pixels around it lie inside the
+// 1-pixel border, so that no pixel, byte or edge needs a check (nine tenths of
+// the tiles of 1920x1080, half of those of 256x256).  EDGE: they do not.  Both:
+// the image's byte offsets fit 32 bits, lambda < 2^22 (q.small) and the image
+// is not constant.  ANY: everything else.
+enum { BUILD_INNER, BUILD_EDGE, BUILD_ANY };
+template <int KIND, int STRIP>
+__device__ __forceinline__ void build_strip(const BuildTile &g, const NlinkParams &q, uint32_t &idp, uint32_t &rinit,
+                                            uint32_t &pos) {
+    constexpr bool INNER = KIND == BUILD_INNER;
+    const int lane = threadIdx.x & 31;
+    const int W = g.W, H = g.H, x = g.x;
+    const uintptr_t lo = (uintptr_t)g.base, hi = lo + 3 * (uintptr_t)W * (uintptr_t)H;
+    const int mis = (int)(lo & 3);
+    const uint8_t *abase = g.base - mis;  // 4-byte aligned
+    // The three aligned words that hold pixel (px, y) and its right neighbour,
+    // and the place of its first byte in them (mod 4).  Where they reach past
+    // the pair they stay inside the image for an inner tile; elsewhere bytes
+    // outside the image, and pixels outside it, read as 0.
+    struct Words {
+        uint32_t w[3];
+        unsigned o;
+    };
+    auto fetch = [&](int px, int y) {
+        Words f;
+        const bool in = INNER || (px >= 0 && px < W && y >= 0 && y < H);
+        if (KIND != BUILD_ANY) {
+            const int o = mis + 3 * (y * W + px), a = o & ~3;
+            const uint8_t *p = abase + a;
+            if (INNER || (in && a >= mis && a + 12 <= mis + 3 * W * H)) {
+#pragma unroll
+                for (int i = 0; i < 3; ++i) f.w[i] = __ldg(reinterpret_cast<const uint32_t *>(p) + i);
+            } else {
+#pragma unroll
+                for (int i = 0; i < 3; ++i) f.w[i] = in ? word_in((uintptr_t)p + 4 * i, lo, hi) : 0u;
+            }
+            f.o = (unsigned)o;
+        } else {
+            const uintptr_t a = in ? lo + 3 * ((uintptr_t)y * W + px) : hi + 4;
+#pragma unroll
+            for (int i = 0; i < 3; ++i) f.w[i] = word_in((a & ~(uintptr_t)3) + 4 * i, lo, hi);
+            f.o = (unsigned)a;
+        }
+        return f;
+    };
+    auto cut = [](const Words &f, uint32_t &c, uint32_t &n) {  // the pair's colours
+        const uint32_t a = __funnelshift_r(f.w[0], f.w[1], f.o * 8), b = __funnelshift_r(f.w[1], f.w[2], f.o * 8);
+        c = a & 0xFFFFFFu;
+        n = __funnelshift_r(a, b, 24) & 0xFFFFFFu;
+    };
+    // Weight of an edge between colours a and b (use: both ends are interior);
+    // bad: the float path leaves it to the double expression.
+    auto weigh = [&](uint32_t a, uint32_t b, bool use, bool &bad) {
+        int w;
+        if (KIND != BUILD_ANY) {
+            bad = !nlink_fast_small(diff2w(a, b), q, w) && (INNER || use);
+            return INNER || use ? w : 0;
+        }
+        bad = false;
+        w = q.const_w;
+        if (!q.constant) bad = use && !nlink_fast(diff2w(a, b), q, w);
+        return use ? w : 0;
+    };
+    auto inside = [&](int px, int y) { return px >= 1 && px <= W - 2 && y >= 1 && y <= H - 2; };
+    const bool col_in = x >= 1 && x <= W - 2, cols_in = x >= 1 && x <= W - 3;  // the lane's and the next column
+
+    constexpr int AHEAD = 3;  // rows of words in flight
+    Words ring[AHEAD + 1];
+    const Words fa = fetch(x, g.ys - 1);
+    const int xl = x - lane - 1;  // the column left of the tile: lane r of 0..7 for row r
+    const Words fl = fetch(xl, g.ys + (lane & (STRIP - 1)));
+#pragma unroll
+    for (int r = 0; r < AHEAD; ++r) ring[r] = fetch(x, g.ys + r);
+    uint32_t c, n;  // this pixel and its right neighbour
+    cut(ring[0], c, n);
+    int wu, wl;  // the edge from above (this row's), from the left (lane r: row r's)
+    {
+        uint32_t a, b;
+        bool bad;
+        cut(fa, a, b);
+        wu = weigh(a, c, inside(x, g.ys - 1) && inside(x, g.ys), bad);
+        if (bad) wu = nlink_exact(diff2w(a, c), q.lambda, q.s2);
+        cut(fl, a, b);
+        const int y = g.ys + (lane & (STRIP - 1));
+        wl = weigh(a, b, inside(xl, y) && inside(xl + 1, y), bad);
+        if (bad) wl = nlink_exact(diff2w(a, b), q.lambda, q.s2);
+    }
+    // the reference sums max(dp, 0) over padded positions x + y * W32 < W * H
+    // (GraphCut.cu:359-376, GraphCutKernels.cu:883-898); 32-bit for an inner tile (W32 < 2 W)
+    const int w32 = (W + 31) & ~31;
+    const int left = INNER ? W * H - x - g.ys * w32 : 0;
+    unsigned mu = __ballot_sync(0xffffffffu, wu > 0);
+#pragma unroll
+    for (int r = 0; r < STRIP; ++r) {
+        const int y = g.ys + r;
+        if (r + AHEAD <= STRIP) ring[(r + AHEAD) % (AHEAD + 1)] = fetch(x, y + AHEAD);
+        uint32_t cd, nd;  // the row below
+        cut(ring[(r + 1) % (AHEAD + 1)], cd, nd);
+        bool bad_r, bad_d;
+        int wr = weigh(c, n, cols_in && y >= 1 && y <= H - 2, bad_r);
+        int wd = weigh(c, cd, col_in && y >= 1 && y <= H - 3, bad_d);
+        if (__any_sync(0xffffffffu, bad_r || bad_d)) {  // rare
+            if (bad_r) wr = nlink_exact(diff2w(c, n), q.lambda, q.s2);
+            if (bad_d) wd = nlink_exact(diff2w(c, cd), q.lambda, q.s2);
+        }
+        const int wl_r = __shfl_sync(0xffffffffu, wl, r);
+        int4 k;
+        k.x = __shfl_up_sync(0xffffffffu, wr, 1);
+        if (lane == 0) k.x = wl_r;
+        k.y = wr;
+        k.z = wu;
+        k.w = wd;
+        int e = 0;
+        if (INNER || (x < W && y < H)) {
+            const int2 v = __ldg(g.lut + color_binw(c));
+            const bool counted = INNER ? r * w32 < left : (long long)x + (long long)y * w32 < (long long)W * H;
+            if (counted) rinit += (unsigned)max(v.x, 0);
+            if (INNER || inside(x, y)) {
+                e = v.x - v.y;
+                idp += (unsigned)v.x;
+            }
+        }
+        g.cap[r * 32] = k;
+        g.exc[r * 32] = e;
+        pos += (unsigned)max(e, 0);
+        // of the six mask planes, the left one is the right one moved by a
+        // column, the upper one the lower one of the row before
+        const unsigned mr = __ballot_sync(0xffffffffu, wr > 0), md = __ballot_sync(0xffffffffu, wd > 0);
+        const unsigned mn = __ballot_sync(0xffffffffu, e < 0), mp = __ballot_sync(0xffffffffu, e > 0);
+        if (lane == 0) {
+            g.msk[0][g.r0 + r] = mr << 1 | (k.x > 0 ? 1u : 0u);
+            g.msk[1][g.r0 + r] = mr;
+            g.msk[2][g.r0 + r] = mu;
+            g.msk[3][g.r0 + r] = md;
+            g.msk[4][g.r0 + r] = mn;
+            g.msk[5][g.r0 + r] = mp;
+        }
+        mu = md;
+        wu = wd;
+        c = cd;
+        n = nd;
+    }
+}
+
+// Strips of 8 rows (4 warps per tile) do the least work per tile; up to
+// BUILD_SMALL_TILES tiles, which are all resident at once, the time is that of
+// one strip, and strips of 4 rows are shorter: 8 against 4 warps 9.7 / 11.9 us
+// for 256x256 (64 tiles), 10.1 / 13.9 for 512x512, 12.2 / 12.5 for 900x900 (841
+// tiles), 20.1 / 19.5 for 1920x1080 (2040), 121 / 96 for 4096x4096.  (2 rows: 8.7
+// for 256x256, 14.3 for 900x900; 16 rows: 100 for 4096x4096, 396 for the batch.)
+constexpr int BUILD_SMALL_TILES = 1024;
+template <int WARPS>
+__global__ void __launch_bounds__(WARPS * 32, 32 / WARPS) k_build_img_b(Batch b, const uint8_t *__restrict__ rgb,
+                                                                   const int2 *__restrict__ tl_lut) {
+    constexpr int STRIP = TILE_H / WARPS;
+    __shared__ uint32_t msk[6][TILE_H];  // mask planes of the tile, stored coalesced below
+    __shared__ unsigned long long wsum[3][WARPS];
     const int t = batch_tile(b, blockIdx.x);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int im = __ldg(b.tile_img + t);
-    const ImgDesc d = b.img[im];
+    const ImgDesc &d = b.img[im];
+    const int W = d.W, H = d.H, tiles_x = d.tiles_x, tiles_y = d.tiles_y;
     const int lt = t - d.tile0;
-    const int tx = lt % d.tiles_x, ty = lt / d.tiles_x;
+    const int ty = lt / tiles_x, tx = lt - ty * tiles_x;
     if (threadIdx.x == 0)  // the tile's neighbours, for the solver
-        b.tile_nb[t] = make_int4(tx > 0 ? t - 1 : -1, tx < d.tiles_x - 1 ? t + 1 : -1, ty > 0 ? t - d.tiles_x : -1,
-                                 ty < d.tiles_y - 1 ? t + d.tiles_x : -1);
-    const int W = d.W, H = d.H;
+        b.tile_nb[t] = make_int4(tx > 0 ? t - 1 : -1, tx < tiles_x - 1 ? t + 1 : -1, ty > 0 ? t - tiles_x : -1,
+                                 ty < tiles_y - 1 ? t + tiles_x : -1);
     const int x0 = tx * TILE_W, y0 = ty * TILE_H;
     const NlinkParams q = nlink_params(d.lambda, b.ist[im]);
-    const int *dpl = dp_lut + (size_t)im * NBINS;
-    const int *dnl = dn_lut + (size_t)im * NBINS;
-    const uint8_t *base = rgb + 3 * d.pix0;
-
-    // Stage the 34 rows of 34 pixels (tile + 1-pixel halo) as packed colours.
-    // Warp w takes rows w, w + 8, ...: the row's bytes are fetched as aligned
-    // 32-bit words, one per lane (at most 27; a word that reaches outside
-    // this image's bytes is assembled from the bytes inside), and each lane
-    // cuts its pixel out of two adjacent words (warp shuffles + a funnel
-    // shift); lanes 0 and 1 then cut the row's last two pixels.
-    if (3LL * W * H < (1LL << 30)) {  // block-uniform: the image's byte offsets fit 32 bits
-        // The same staging with 32-bit offsets from the 4-byte-aligned
-        // address at or below the image's first byte (mis = the image's
-        // misalignment): 64-bit address arithmetic costs several
-        // instructions per operation, and every thread runs it per row.
-        const uintptr_t lo = (uintptr_t)base;
-        const int mis = (int)(lo & 3);
-        const uint8_t *abase = base - mis;  // 4-byte aligned
-        const int nbytes = 3 * W * H;
-        const int xs = x0 > 0 ? x0 - 1 : 0;
-        const int xe = x0 + TILE_W < W ? x0 + TILE_W : W - 1;
-        constexpr int NW = TILE_THREADS / 32, RPW = (SH + NW - 1) / NW;  // rows per warp
-        uint32_t words[RPW];
-        int phs[RPW];
-#pragma unroll
-        for (int r = 0; r < RPW; ++r) {  // every load first
-            const int i = warp + NW * r;
-            const int y = y0 - 1 + i;
-            uint32_t word = 0;
-            const int rs = mis + 3 * (y * W + xs);  // aligned-base offset of the row's first byte
-            phs[r] = rs & 3;
-            if (i < SH && y >= 0 && y < H) {
-                const int re = mis + 3 * (y * W + xe) + 3;  // one past its last byte
-                const int aw = rs & ~3;
-                if (lane < ((re - aw + 3) >> 2)) {
-                    const int wa = aw + 4 * lane;   // aligned-base offset of the lane's word
-                    const int k0 = wa - mis;        // image byte offset of its first byte
-                    if (k0 >= 0 && k0 + 4 <= nbytes) {
-                        word = __ldg(reinterpret_cast<const uint32_t *>(abase + wa));
-                    } else {
-#pragma unroll
-                        for (int k = 0; k < 4; ++k)
-                            if (k0 + k >= 0 && k0 + k < nbytes) word |= (uint32_t)__ldg(abase + wa + k) << (8 * k);
-                    }
-                }
-            }
-            words[r] = word;
-        }
-#pragma unroll
-        for (int r = 0; r < RPW; ++r) {
-            const int i = warp + NW * r;
-            if (i >= SH) break;  // warp-uniform
-            const int y = y0 - 1 + i;
-            const bool row_in = y >= 0 && y < H;
-            const int ph = phs[r];
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int j = lane + 32 * h;
-                const int x = x0 - 1 + j;
-                const bool in = row_in && x >= 0 && x < W;
-                const int off = in ? ph + 3 * (x - xs) : 0;  // <= 3 + 3 * 33 = 102: words 0..26
-                const uint32_t wlo = __shfl_sync(0xffffffffu, words[r], off >> 2);
-                const uint32_t whi = __shfl_sync(0xffffffffu, words[r], (off >> 2) + 1);
-                const uint32_t v = in ? __funnelshift_r(wlo, whi, (off & 3) * 8) & 0xFFFFFFu : 0u;
-                if (j < SW) col[i][j] = v;
-            }
-        }
-    } else {
-        const uintptr_t lo = (uintptr_t)base, hi = lo + 3 * (uintptr_t)W * (uintptr_t)H;
-        const int xs = x0 > 0 ? x0 - 1 : 0;
-        const int xe = x0 + TILE_W < W ? x0 + TILE_W : W - 1;
-        constexpr int NW = TILE_THREADS / 32, RPW = (SH + NW - 1) / NW;  // rows per warp
-        uint32_t words[RPW];
-#pragma unroll
-        for (int r = 0; r < RPW; ++r) {  // every load first
-            const int i = warp + NW * r;
-            const int y = y0 - 1 + i;
-            uint32_t word = 0;
-            if (i < SH && y >= 0 && y < H) {
-                const uintptr_t a0 = lo + 3 * ((uintptr_t)y * W + xs);
-                const uintptr_t a1 = lo + 3 * ((uintptr_t)y * W + xe) + 3;
-                const uintptr_t aw = a0 & ~(uintptr_t)3;
-                if (lane < (int)((a1 - aw + 3) >> 2)) {
-                    const uintptr_t wa = aw + 4 * (uintptr_t)lane;
-                    if (wa >= lo && wa + 4 <= hi) {
-                        word = __ldg(reinterpret_cast<const uint32_t *>(wa));
-                    } else {
-#pragma unroll
-                        for (int k = 0; k < 4; ++k)
-                            if (wa + k >= lo && wa + k < hi)
-                                word |= (uint32_t)__ldg(reinterpret_cast<const uint8_t *>(wa + k)) << (8 * k);
-                    }
-                }
-            }
-            words[r] = word;
-        }
-#pragma unroll
-        for (int r = 0; r < RPW; ++r) {
-            const int i = warp + NW * r;
-            if (i >= SH) break;  // warp-uniform
-            const int y = y0 - 1 + i;
-            const bool row_in = y >= 0 && y < H;
-            const int ph = (int)((lo + 3 * ((uintptr_t)y * W + xs)) & 3);  // first byte's place in its word
-            // pixel j = lane (x = x0 - 1 + lane), then j = 32 + lane for lanes 0, 1
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int j = lane + 32 * h;
-                const int x = x0 - 1 + j;
-                const bool in = row_in && x >= 0 && x < W;
-                const int off = in ? ph + 3 * (x - xs) : 0;  // <= 3 + 3 * 33 = 102: words 0..26
-                const uint32_t wlo = __shfl_sync(0xffffffffu, words[r], off >> 2);
-                const uint32_t whi = __shfl_sync(0xffffffffu, words[r], (off >> 2) + 1);
-                const uint32_t v = in ? __funnelshift_r(wlo, whi, (off & 3) * 8) & 0xFFFFFFu : 0u;
-                if (j < SW) col[i][j] = v;
-            }
-        }
-    }
-    __syncthreads();
-    // 2048 edges inside the tile's rows and columns, 8 per thread (right
-    // edges wr[i][1..32], then down edges wd[1..32][j]), and the 64 edges
-    // that reach into the tile from the left and from above (wr[i][0], wd[0][j])
-    {
-        // thread (warp, lane): right edges of pixel (x0 + lane, y0 + warp + 8u),
-        // u = 0..3, and down edges of the same pixels, u = 4..7
-        constexpr int PER = 2 * TILE_W * TILE_H / TILE_THREADS;
-        static_assert(PER == 8 && ROWS_PER_WARP == 4, "edge split assumes 8 warps of 32 lanes");
-        const int x = x0 + lane;
-        const bool xr = x >= 1 && x <= W - 3, xd = x >= 1 && x <= W - 2;
-        // each weight goes to shared memory as soon as it is known; the rare
-        // ones within the margin of a rounding boundary are redone exactly
-        unsigned exact = 0;  // bit u: edge u needs the double expression
-#pragma unroll
-        for (int u = 0; u < PER; ++u) {
-            const int i = warp + 8 * (u & 3);
-            const int y = y0 + i;
-            bool use;
-            int d2;
-            if (u < 4) {
-                use = xr && y >= 1 && y <= H - 2;
-                d2 = diff2w(col[i + 1][lane + 1], col[i + 1][lane + 2]);
-            } else {
-                use = xd && y >= 1 && y <= H - 3;
-                d2 = diff2w(col[i + 1][lane + 1], col[i + 2][lane + 1]);
-            }
-            int w = 0;
-            if (q.constant) {
-                w = q.const_w;
-            } else if (!nlink_fast(d2, q, w)) {
-                exact |= 1u << u;
-            }
-            if (!use) {
-                w = 0;
-                exact &= ~(1u << u);
-            }
-            if (u < 4) wr[i][lane + 1] = w;
-            else wd[i + 1][lane] = w;
-        }
-        if (__any_sync(0xffffffffu, exact != 0)) {
-            for (unsigned m = exact; m; m &= m - 1) {
-                const int u = __ffs(m) - 1;
-                const int i = warp + 8 * (u & 3);
-                if (u < 4) wr[i][lane + 1] = nlink_exact(diff2w(col[i + 1][lane + 1], col[i + 1][lane + 2]), q.lambda, q.s2);
-                else wd[i + 1][lane] = nlink_exact(diff2w(col[i + 1][lane + 1], col[i + 2][lane + 1]), q.lambda, q.s2);
-            }
-        }
-        if (threadIdx.x < 2 * 32) {
-            const int j = threadIdx.x & 31;
-            int w = 0;
-            if (threadIdx.x < 32) {  // edge (x0 - 1, y0 + j)-(x0, y0 + j)
-                const int x = x0 - 1, y = y0 + j;
-                if (x >= 1 && x <= W - 3 && y >= 1 && y <= H - 2) w = nlink_w(diff2w(col[j + 1][0], col[j + 1][1]), q);
-                wr[j][0] = w;
-            } else {  // edge (x0 + j, y0 - 1)-(x0 + j, y0)
-                const int x = x0 + j, y = y0 - 1;
-                if (y >= 1 && y <= H - 3 && x >= 1 && x <= W - 2) w = nlink_w(diff2w(col[0][j + 1], col[1][j + 1]), q);
-                wd[0][j] = w;
-            }
-        }
-    }
-    __syncthreads();
-
-    // Per pixel (thread (warp, lane), rows warp + 8k): capacities, excess and
-    // the sums of the tile.  Per-thread sums stay below 2^30 (4 pixels of at
-    // most GCFG_MAX_CAP), so they are 32-bit and each warp adds them exactly
-    // with two 32-bit reductions of their 16-bit halves.
-    __shared__ uint32_t msk[6][TILE_H];  // mask planes of the tile, stored coalesced below
-    __shared__ unsigned long long wsum[3][TILE_THREADS / 32];
-    const long long w32 = (long long)((W + 31) / 32) * 32, npx = (long long)W * H;
-    const int x = x0 + lane;
+    BuildTile g;
+    g.W = W;
+    g.H = H;
+    g.x = x0 + lane;
+    g.r0 = STRIP * warp;
+    g.ys = y0 + g.r0;
+    g.base = rgb + 3 * d.pix0;
+    g.lut = tl_lut + (size_t)im * NBINS;
+    g.cap = b.cap + (size_t)t * TPX + g.r0 * 32 + lane;
+    g.exc = b.exc + (size_t)t * TPX + g.r0 * 32 + lane;
+    g.msk = msk;
     uint32_t idp = 0, rinit = 0, pos = 0;
-    int4 *cap = b.cap + (size_t)t * TPX;
-    int *exc = b.exc + (size_t)t * TPX;
-#pragma unroll
-    for (int k = 0; k < ROWS_PER_WARP; ++k) {
-        const int r = warp + 8 * k;
-        const int y = y0 + r;
-        int4 c = make_int4(0, 0, 0, 0);
-        int e = 0;
-        if (x < W && y < H) {
-            const int bin = color_binw(col[r + 1][lane + 1]);
-            const int vdp = __ldg(dpl + bin);
-            if ((long long)x + (long long)y * w32 < npx && vdp > 0) rinit += (unsigned)vdp;
-            if (x > 0 && y > 0 && x < W - 1 && y < H - 1) {
-                c.x = wr[r][lane];      // left: edge (x - 1, y)-(x, y)
-                c.y = wr[r][lane + 1];  // right
-                c.z = wd[r][lane];      // up: edge (x, y - 1)-(x, y)
-                c.w = wd[r + 1][lane];  // down
-                e = vdp - __ldg(dnl + bin);
-                idp += (unsigned)vdp;
-            }
-        }
-        cap[r * 32 + lane] = c;
-        exc[r * 32 + lane] = e;
-        const unsigned ml = __ballot_sync(0xffffffffu, c.x > 0);
-        const unsigned mr = __ballot_sync(0xffffffffu, c.y > 0);
-        const unsigned mu = __ballot_sync(0xffffffffu, c.z > 0);
-        const unsigned md = __ballot_sync(0xffffffffu, c.w > 0);
-        const unsigned mn = __ballot_sync(0xffffffffu, e < 0);
-        const unsigned mp = __ballot_sync(0xffffffffu, e > 0);
-        if (lane == 0) {
-            msk[0][r] = ml; msk[1][r] = mr; msk[2][r] = mu; msk[3][r] = md; msk[4][r] = mn; msk[5][r] = mp;
-        }
-        if (e > 0) pos += (unsigned)e;
-    }
+    if (3LL * W * H >= (1LL << 30) || !q.small || q.constant)
+        build_strip<BUILD_ANY, STRIP>(g, q, idp, rinit, pos);
+    else if (tx > 0 && ty > 0 && x0 + TILE_W + 1 < W && y0 + TILE_H + 1 < H)
+        build_strip<BUILD_INNER, STRIP>(g, q, idp, rinit, pos);
+    else
+        build_strip<BUILD_EDGE, STRIP>(g, q, idp, rinit, pos);
+    // Per-thread sums stay below 2^31 (8 pixels of at most GCFG_MAX_CAP), so
+    // they are 32-bit and each warp adds them exactly with two 32-bit
+    // reductions of their 16-bit halves.
     {
         const uint32_t v[3] = {idp, rinit, pos};
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
-            const unsigned long long lo = __reduce_add_sync(0xffffffffu, v[k] & 0xFFFFu);
-            const unsigned long long hi = __reduce_add_sync(0xffffffffu, v[k] >> 16);
-            if (lane == 0) wsum[k][warp] = (hi << 16) + lo;
+            const unsigned long long l = __reduce_add_sync(0xffffffffu, v[k] & 0xFFFFu);
+            const unsigned long long h = __reduce_add_sync(0xffffffffu, v[k] >> 16);
+            if (lane == 0) wsum[k][warp] = (h << 16) + l;
         }
     }
     __syncthreads();
-    if (threadIdx.x < 6 * TILE_H)
-        b.tmask[(size_t)t * 6 * 32 + threadIdx.x] = msk[threadIdx.x >> 5][threadIdx.x & 31];
+    for (int i = threadIdx.x; i < 6 * TILE_H; i += WARPS * 32)
+        b.tmask[(size_t)t * 6 * 32 + i] = msk[i >> 5][i & 31];
     if (warp == 0) {
         // lanes 0..2: the tile's three sums
         unsigned long long tot = 0;
         if (lane < 3)
-            for (int w8 = 0; w8 < TILE_THREADS / 32; ++w8) tot += wsum[lane][w8];
+            for (int w = 0; w < WARPS; ++w) tot += wsum[lane][w];
         if (lane == 0 && tot) atomicAdd(&b.ist[im].interior_dp, tot);
         if (lane == 1 && tot) atomicAdd(&b.ist[im].ref_init, tot);
         if (lane == 2) b.tile_pos[t] = tot;
@@ -762,13 +730,13 @@ __global__ void __launch_bounds__(TILE_THREADS, 8) k_build_img_b(Batch b, const 
 
 // Row-major t-link / n-link arrays of image 0 (the stand-alone data-term API).
 __global__ void k_tlinks_apply(const uint8_t *__restrict__ rgb, long long n,
-                               const int *__restrict__ dp_lut, const int *__restrict__ dn_lut,
-                               int *__restrict__ dp, int *__restrict__ dn) {
+                               const int2 *__restrict__ tl_lut, int *__restrict__ dp, int *__restrict__ dn) {
     const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (i >= n) return;
     const int bin = color_bin3(rgb + 3 * i);
-    dp[i] = __ldg(dp_lut + bin);
-    dn[i] = __ldg(dn_lut + bin);
+    const int2 v = __ldg(tl_lut + bin);
+    dp[i] = v.x;
+    dn[i] = v.y;
 }
 
 // One block per 32 x 32 pixels, thread (x, y) four rows of column x.  Each
@@ -826,7 +794,7 @@ gcfg_status dt_tables(const DtArgs &a, cudaStream_t st) {
                                                                a.ist));
     if (a.scrib)
         GCFG_LAUNCH(GCFG_PK_TLUT, st,
-                    k_tlut_b<<<a.n_img, 1024, 0, st>>>(a.ilist, a.hist, a.img, a.ist, a.dp_lut, a.dn_lut, a.raw_dp,
+                    k_tlut_b<<<a.n_img, 1024, 0, st>>>(a.ilist, a.hist, a.img, a.ist, a.tl_lut, a.raw_dp,
                                                        a.raw_dn));
     else
         GCFG_LAUNCH(GCFG_PK_TLUT, st,
@@ -836,15 +804,18 @@ gcfg_status dt_tables(const DtArgs &a, cudaStream_t st) {
 }
 
 gcfg_status dt_build(const Batch &b, const DtArgs &a, cudaStream_t st) {
-    GCFG_LAUNCH(GCFG_PK_BUILD, st,
-                k_build_img_b<<<batch_ntiles(b), TILE_THREADS, 0, st>>>(b, a.rgb, a.dp_lut, a.dn_lut));
+    const int tiles = batch_ntiles(b);
+    if (tiles <= BUILD_SMALL_TILES)
+        GCFG_LAUNCH(GCFG_PK_BUILD, st, k_build_img_b<8><<<tiles, 256, 0, st>>>(b, a.rgb, a.tl_lut));
+    else
+        GCFG_LAUNCH(GCFG_PK_BUILD, st, k_build_img_b<4><<<tiles, 128, 0, st>>>(b, a.rgb, a.tl_lut));
     GCFG_CK(cudaGetLastError());
     return GCFG_OK;
 }
 
 gcfg_status dt_apply_tlinks(const DtArgs &a, long long n, int *dp, int *dn, cudaStream_t st) {
     GCFG_LAUNCH(GCFG_PK_OTHER, st,
-                k_tlinks_apply<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(a.rgb, n, a.dp_lut, a.dn_lut, dp, dn));
+                k_tlinks_apply<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(a.rgb, n, a.tl_lut, dp, dn));
     GCFG_CK(cudaGetLastError());
     return GCFG_OK;
 }

@@ -23,7 +23,7 @@ inline long long max_chunks(long long n, long long px) { return px / CHUNK_PX + 
 inline long long image_chunks(int W, int H, int chunk) { return ((long long)W * H + chunk - 1) / chunk; }
 
 // Device buffers of the data term for a batch (per image: 2*4096 histogram
-// bins, 4096 dp and dn entries).
+// bins, 4096 (dp, dn) entries).
 struct DtArgs {
     int n_img;                // images of this pass (local index k)
     const int *ilist;         // local image k -> image (slot) index; NULL: k itself
@@ -35,7 +35,7 @@ struct DtArgs {
     const int2 *chunk_map;    // per chunk of the pass: (image index, chunk index within the image)
     int chunk;                // pixels per chunk
     int *hist;
-    int *dp_lut, *dn_lut;
+    int2 *tl_lut;             // per bin the t-links (dp, dn): one 8-byte gather per pixel
     double *raw_dp, *raw_dn;  // optional (NULL): pre-rounding per-bin values
 };
 

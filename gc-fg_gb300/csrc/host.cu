@@ -65,7 +65,7 @@ struct Engine {
     ImgDesc *d_img = nullptr;
     int2 *d_cmap = nullptr;    // per chunk of the data-term pass: (image, chunk in image)
     int *d_tile_img = nullptr;
-    int *d_dpl = nullptr, *d_dnl = nullptr;
+    int2 *d_lut = nullptr;
     int4 *d_cap = nullptr;
     int *d_exc = nullptr, *d_h = nullptr, *d_hb = nullptr;
     int4 *d_tnb = nullptr;
@@ -266,8 +266,7 @@ struct Engine {
         c.put(d_img, cap_imgs);
         c.put(d_cmap, cap_chunks);
         c.put(d_tile_img, T);
-        c.put(d_dpl, cap_dt ? cap_imgs * NBINS : 0);
-        c.put(d_dnl, cap_dt ? cap_imgs * NBINS : 0);
+        c.put(d_lut, cap_dt ? cap_imgs * NBINS : 0);
         c.put(d_cap, T * TPX);
         c.put(d_exc, T * TPX);
         c.put(d_h, T * TPX);
@@ -528,8 +527,7 @@ struct Engine {
         a.chunk_map = d_cmap;
         a.chunk = chunk;
         a.hist = d_hist;
-        a.dp_lut = d_dpl;
-        a.dn_lut = d_dnl;
+        a.tl_lut = d_lut;
         a.raw_dp = nullptr;
         a.raw_dn = nullptr;
         return a;
@@ -759,7 +757,8 @@ namespace {
 struct OneImage {
     char *slab = nullptr;
     ImgState *ist = nullptr;
-    int *hist = nullptr, *dpl = nullptr, *dnl = nullptr;
+    int *hist = nullptr;
+    int2 *lut = nullptr;
     ImgDesc *img = nullptr;
     double *raw = nullptr;
     ImgDesc desc;  // the host's copy: alive until the stream is synchronised
@@ -770,8 +769,7 @@ struct OneImage {
         c.put(ist, 1);
         c.put(hist, with_hist ? 2 * NBINS : 0);
         c.put(img, 1);
-        c.put(dpl, with_hist ? NBINS : 0);
-        c.put(dnl, with_hist ? NBINS : 0);
+        c.put(lut, with_hist ? NBINS : 0);
         c.put(raw, with_raw ? 2 * NBINS : 0);
         return c.off;
     }
@@ -800,8 +798,7 @@ struct OneImage {
         a.img = img;
         a.ist = ist;
         a.hist = hist;
-        a.dp_lut = dpl;
-        a.dn_lut = dnl;
+        a.tl_lut = lut;
         a.raw_dp = with_raw ? raw : nullptr;
         a.raw_dn = with_raw ? raw + NBINS : nullptr;
         return dt_tables(a, st);

@@ -148,9 +148,8 @@ __global__ void k_edit_square(uint8_t *scrib, int W, int H, int x0, int y0, int 
 // Warm start: shift every interior pixel's excess by the change of its
 // t-links, keep capacities, refresh the mask planes and the image sums.
 __global__ void __launch_bounds__(TILE_THREADS) k_reparam(Batch b, const uint8_t *__restrict__ rgb,
-                                                           const int *__restrict__ dpl, const int *__restrict__ dnl,
-                                                           const int *__restrict__ odpl,
-                                                           const int *__restrict__ odnl) {
+                                                           const int2 *__restrict__ lut,
+                                                           const int2 *__restrict__ olut) {
     const int t = batch_tile(b, blockIdx.x);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int im = b.tile_img[t];
@@ -172,10 +171,12 @@ __global__ void __launch_bounds__(TILE_THREADS) k_reparam(Batch b, const uint8_t
         if (x < W && y < H) {
             const uint8_t *p = base + 3 * ((long long)y * W + x);
             const int bin = ((p[0] >> 4) << 8) | ((p[1] >> 4) << 4) | (p[2] >> 4);
-            const int vdp = dpl[lo + bin];
+            const int2 v = lut[lo + bin];
+            const int vdp = v.x;
             if ((long long)x + (long long)y * w32 < (long long)W * H && vdp > 0) rinit += (unsigned)vdp;
             if (x > 0 && y > 0 && x < W - 1 && y < H - 1) {
-                e += (vdp - odpl[lo + bin]) - (dnl[lo + bin] - odnl[lo + bin]);
+                const int2 o = olut[lo + bin];
+                e += (vdp - o.x) - (v.y - o.y);
                 b.exc[q] = e;
                 idp += (unsigned)vdp;
             }
@@ -209,7 +210,8 @@ struct Server {
     // slots
     ImgDesc *img = nullptr;
     ImgState *ist = nullptr;
-    int *hist = nullptr, *dpl = nullptr, *dnl = nullptr, *odpl = nullptr, *odnl = nullptr;
+    int *hist = nullptr;
+    int2 *lut = nullptr, *olut = nullptr;  // t-link tables, and those before the last edit
     // host state
     std::mutex mu;
     std::condition_variable cv_work, cv_done;
@@ -361,10 +363,8 @@ gcfg_status run_batch(Lane &L, std::vector<Req> &batch, const std::vector<Sessio
             GCFG_CK(cudaMemcpyAsync(s.scrib + x.pix0, batch[k].r.h_scrib, npx, cudaMemcpyHostToDevice, st));
         } else {
             // keep the current tables as the "previous" ones, then edit the scribbles
-            GCFG_CK(cudaMemcpyAsync(s.odpl + (size_t)x.slot * NBINS, s.dpl + (size_t)x.slot * NBINS,
-                                    NBINS * sizeof(int), cudaMemcpyDeviceToDevice, st));
-            GCFG_CK(cudaMemcpyAsync(s.odnl + (size_t)x.slot * NBINS, s.dnl + (size_t)x.slot * NBINS,
-                                    NBINS * sizeof(int), cudaMemcpyDeviceToDevice, st));
+            GCFG_CK(cudaMemcpyAsync(s.olut + (size_t)x.slot * NBINS, s.lut + (size_t)x.slot * NBINS,
+                                    NBINS * sizeof(int2), cudaMemcpyDeviceToDevice, st));
             const int sz = batch[k].r.edit_size;
             dim3 blk(16, 16), grd(div_up(sz, 16), div_up(sz, 16));
             k_edit_square<<<grd, blk, 0, st>>>(s.scrib + x.pix0, x.W, x.H, batch[k].r.edit_x, batch[k].r.edit_y, sz,
@@ -393,8 +393,7 @@ gcfg_status run_batch(Lane &L, std::vector<Req> &batch, const std::vector<Sessio
     a.chunk_map = L.d_cmap;
     a.chunk = chunk;
     a.hist = s.hist;
-    a.dp_lut = s.dpl;
-    a.dn_lut = s.dnl;
+    a.tl_lut = s.lut;
     for (int k = 0; k < n; ++k)
         GCFG_CK(cudaMemsetAsync(s.hist + (size_t)L.h_il[k] * 2 * NBINS, 0, 2 * NBINS * sizeof(int), st));
     GCFG_TRY(dt_tables(a, st));
@@ -413,7 +412,7 @@ gcfg_status run_batch(Lane &L, std::vector<Req> &batch, const std::vector<Sessio
         Batch be = b;
         be.tlist = L.d_tedit;
         be.n_tlist = nedit;
-        k_reparam<<<nedit, TILE_THREADS, 0, st>>>(be, s.rgb, s.dpl, s.dnl, s.odpl, s.odnl);
+        k_reparam<<<nedit, TILE_THREADS, 0, st>>>(be, s.rgb, s.lut, s.olut);
         g_launches.fetch_add(1, std::memory_order_relaxed);
         GCFG_CK(cudaGetLastError());
     }
@@ -584,8 +583,8 @@ void shutdown_server(Server *s) {
     cudaFree(s->cap); cudaFree(s->exc); cudaFree(s->h); cudaFree(s->hb); cudaFree(s->tnb); cudaFree(s->hfin); cudaFree(s->reach); cudaFree(s->tmask); cudaFree(s->tact);
     cudaFree(s->tpos); cudaFree(s->mpush); cudaFree(s->mgr); cudaFree(s->tile_img);
     cudaFree(s->rgb); cudaFree(s->scrib); cudaFree(s->smin); cudaFree(s->smax);
-    cudaFree(s->img); cudaFree(s->ist); cudaFree(s->hist); cudaFree(s->dpl); cudaFree(s->dnl);
-    cudaFree(s->odpl); cudaFree(s->odnl);
+    cudaFree(s->img); cudaFree(s->ist); cudaFree(s->hist); cudaFree(s->lut);
+    cudaFree(s->olut);
 }
 
 }  // namespace
@@ -621,8 +620,7 @@ gcfg_status gcfg_serve_create(const gcfg_serve_config *cfg, gcfg_server **out) {
     chk(dalloc(s->rgb, 3 * (size_t)s->px_cap)); chk(dalloc(s->scrib, (size_t)s->px_cap));
     chk(dalloc(s->smin, (size_t)s->px_cap)); chk(dalloc(s->smax, (size_t)s->px_cap));
     chk(dalloc(s->img, NS)); chk(dalloc(s->ist, NS)); chk(dalloc(s->hist, NS * 2 * NBINS));
-    chk(dalloc(s->dpl, NS * NBINS)); chk(dalloc(s->dnl, NS * NBINS));
-    chk(dalloc(s->odpl, NS * NBINS)); chk(dalloc(s->odnl, NS * NBINS));
+    chk(dalloc(s->lut, NS * NBINS)); chk(dalloc(s->olut, NS * NBINS));
     if (rc == GCFG_OK) {
         // every slot starts "solved" so that solves of other slots skip it
         std::vector<ImgState> init(NS);
