@@ -65,13 +65,16 @@ __device__ __noinline__ double tlink_raw(int h, long long N) {
 
 // round(10 * -ln((h+1)/N)).  Float error: the ratio carries <= 3 ulp
 // (conversions and division, 1.8e-7 relative), which moves the log by
-// <= 1.8e-7; logf adds <= 1 ulp of a result <= 22 (2.7e-6); times 10:
-// < 3e-5.  Margin used: 1e-3.
+// <= 1.8e-7; logf adds <= 1 ulp of a result <= 22 (1.9e-6); times 10, and
+// half an ulp of the product (7.6e-6): < 3e-5.  Margin used: 1e-4, as a warp
+// with one entry inside it runs the double expression on a pipe of two lanes
+// per SM and cycle, which bounds the tables' kernel: 256 images 36 us with
+// a margin of 1e-3, 18 with 1e-4.
 __device__ __forceinline__ int tlink_quant(int h, long long N) {
     const float pf = (float)(h + 1) / (float)N;
     const float v = -10.0f * logf(pf);
     const float fr = v - floorf(v);
-    if (fabsf(fr - 0.5f) > 1e-3f) return (int)floorf(v + 0.5f);
+    if (fabsf(fr - 0.5f) > 1e-4f) return (int)floorf(v + 0.5f);
     return (int)round(tlink_raw(h, N));
 }
 
@@ -225,7 +228,7 @@ template <int WS>
 __device__ __forceinline__ uint32_t sigma_chunk(uintptr_t lo, uintptr_t hi, uintptr_t c0, uintptr_t aw, int nvec,
                                                 uintptr_t vstep, int bs, int kh, int kv, uint4 *keep) {
     const int lane = threadIdx.x & 31;
-    uint32_t acc = 0;  // at most 4 vectors of 32 pairs of 65025 per thread
+    uint32_t acc = 0;  // at most 7 vectors of 32 pairs of 65025 per thread
     for (int v0 = (int)threadIdx.x - lane; v0 < nvec; v0 += blockDim.x) {  // warp-uniform trip count
         const int vi = v0 + lane;
         const uintptr_t a = aw + 16 * (uintptr_t)vi;
@@ -276,12 +279,17 @@ __device__ __forceinline__ uint32_t sigma_chunk(uintptr_t lo, uintptr_t hi, uint
                     dh &= byte_mask(o + 4 * j, 0, kh);
                     dv &= byte_mask(o + 4 * j, 0, kv);
                 }
-                acc += __dp4a(dh, dh, 0u) + __dp4a(dv, dv, 0u);
+                acc = __dp4a(dv, dv, __dp4a(dh, dh, acc));
             }
         }
     }
     return acc;
 }
+
+// Shared memory of a block for its chunk: no more than it needs, as what is
+// left of the SM's is the L1 cache that serves the rows below (4096x4096, chunks
+// of 4096 pixels: 46 us with 12 KB per block, 48 with 24).
+inline size_t hist_smem(int chunk) { return ((3 * (size_t)chunk + 15) / 16 + 1) * sizeof(uint4); }
 
 // One pass over a chunk of an image (`chunk` consecutive pixels, row-major):
 // the exact sum of ||dI||^2 over right and down neighbour pairs (for sigma^2)
@@ -302,7 +310,7 @@ __global__ void __launch_bounds__(256, 8) k_hist_sigma_b(const uint8_t *__restri
                                                       const ImgDesc *__restrict__ img,
                                                       const int2 *__restrict__ chunk_map, int chunk,
                                                       int *__restrict__ hist, ImgState *ist) {
-    __shared__ uint4 keep[(3 * CHUNK_PX + 15) / 16 + 1];  // the chunk's bytes from its 16-aligned start
+    extern __shared__ uint4 keep[];  // the chunk's bytes from its 16-aligned start (hist_smem)
     // (image, chunk within the image); no map: one image
     const int2 cm = chunk_map ? __ldg(chunk_map + blockIdx.x) : make_int2(0, (int)blockIdx.x);
     const int im = cm.x;
@@ -373,7 +381,12 @@ __global__ void __launch_bounds__(256, 8) k_hist_sigma_b(const uint8_t *__restri
         for (int v0 = (int)threadIdx.x - lane; v0 < nsw; v0 += blockDim.x) {
             const int vi = v0 + lane;
             const uintptr_t a = saw + 4 * (uintptr_t)vi;
-            const uint32_t w = vi < nsw ? word_in(a, slo, shi) : 0u;
+            uint32_t w;
+            if (saw + 4 * (uintptr_t)v0 >= slo && saw + 4 * (uintptr_t)(v0 + 32) <= shi)  // warp-uniform
+                w = __ldg(reinterpret_cast<const uint32_t *>(a));
+            else
+                w = vi < nsw ? word_in(a, slo, shi) : 0u;
+            if (!__any_sync(0xffffffffu, w != 0)) continue;  // most of the image
             const int o = (int)(a - s0);  // chunk pixel of the word's byte 0
             // bit b: byte b is 1 or 2 and lies in the chunk
             unsigned todo = 0;
@@ -790,8 +803,8 @@ gcfg_status dt_tables(const DtArgs &a, cudaStream_t st) {
     // a.scrib == NULL: n-link constants only (the colour histograms need
     // scribbles); the caller has cleared the histograms
     GCFG_LAUNCH(GCFG_PK_HIST, st,
-                k_hist_sigma_b<<<a.total_chunks, 256, 0, st>>>(a.rgb, a.scrib, a.img, a.chunk_map, a.chunk, a.hist,
-                                                               a.ist));
+                k_hist_sigma_b<<<a.total_chunks, 256, hist_smem(a.chunk), st>>>(a.rgb, a.scrib, a.img, a.chunk_map,
+                                                                                a.chunk, a.hist, a.ist));
     if (a.scrib)
         GCFG_LAUNCH(GCFG_PK_TLUT, st,
                     k_tlut_b<<<a.n_img, 1024, 0, st>>>(a.ilist, a.hist, a.img, a.ist, a.tl_lut, a.raw_dp,

@@ -15,11 +15,17 @@ constexpr int NBINS = 4096;                   // 16^3 colour bins per class
 // events, launch included): 256x256 8.6 / 11.0 / 12.7 us, 900x900 12.2 / 11.3 /
 // 14.9, 1920x1080 16.4 / 14.8 / 16.8, 4096x4096 80 / 61 / 46; extraction
 // 6.1 / 6.1 / 6.1, 6.1 / 6.1 / 6.1, 8.2 / 7.2 / 6.5, 25 / 18 / 14.
-constexpr int CHUNK_PX = 4096;  // the largest chunk
-inline int chunk_px_for(long long px) { return px <= (1 << 18) ? 1024 : px <= (1 << 22) ? 2048 : CHUNK_PX; }
+// 4K / 8K: 4096x4096 46 / 49, 256 uneven images of 47 million pixels 116 / 108,
+// their extraction 41 / 37.
+constexpr int CHUNK_PX = 8192;  // the largest chunk
+inline int chunk_px_for(long long px) {
+    return px <= (1 << 18) ? 1024 : px <= (1 << 22) ? 2048 : px <= (1 << 24) ? 4096 : CHUNK_PX;
+}
 // Chunks of any pass of at most n images and px pixels, whatever its own size
-// (a pass of fewer pixels may have smaller chunks).
-inline long long max_chunks(long long n, long long px) { return px / CHUNK_PX + (1 << 22) / 2048 + n + 1; }
+// (a pass of fewer pixels may have smaller chunks: p <= 2^24 pixels make
+// p / 4096 <= p / CHUNK_PX + 2048 of them, and p <= 2^22 at most 2048).
+static_assert(CHUNK_PX == 8192, "max_chunks");
+inline long long max_chunks(long long n, long long px) { return px / CHUNK_PX + 2048 + n + 1; }
 inline long long image_chunks(int W, int H, int chunk) { return ((long long)W * H + chunk - 1) / chunk; }
 
 // Device buffers of the data term for a batch (per image: 2*4096 histogram

@@ -59,3 +59,26 @@ def test_segment_in_each_chunk_size(w, h):
     ref = O.segment(rgb, scrib, 50.0)
     assert res["flow"] == ref["flow"]
     assert np.array_equal(smin, ref["smin"]) and np.array_equal(smax, ref["smax"])
+
+
+def test_terms_in_the_largest_chunks():
+    """More than 2^24 pixels."""
+    test_terms(4111, 4099, "sparse")
+
+
+@pytest.mark.parametrize("n", [1, 7, 97, 1000, 4099, 70001, 999983])
+def test_tlinks_near_rounding_ties(n):
+    """Tables of images of one colour and of two: their entries 10 ln(N / k)
+    take all places between two integers."""
+    import gcfg
+    import oracle as O
+    from gpu_util import dev
+
+    rgb = np.full((n, 1, 3), 40, np.uint8)
+    rgb[: n // 3] = 200
+    scrib = np.full((n, 1), 1, np.uint8)
+    scrib[::2] = 2
+    dp, dn = [torch.zeros((n, 1), dtype=torch.int32, device="cuda") for _ in range(2)]
+    gcfg.tlinks(dev(rgb), dev(scrib), dp, dn)
+    odp, odn = O.tlinks(rgb, scrib)
+    assert np.array_equal(dp.cpu().numpy(), odp) and np.array_equal(dn.cpu().numpy(), odn)
