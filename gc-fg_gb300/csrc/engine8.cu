@@ -172,11 +172,6 @@ constexpr int T8W = 32, T8H = 8;
 #ifndef GCFG_N8_SWEEPS
 #define GCFG_N8_SWEEPS 8    // sweeps per tile visit
 #endif
-__device__ __forceinline__ void red_shared_if(int *p, int v) {  // *p += v, nothing when v is 0
-    const unsigned a = (unsigned)__cvta_generic_to_shared(p);
-    asm volatile("{\n .reg .pred q;\n setp.ne.s32 q, %1, 0;\n @q red.shared.add.s32 [%0], %1;\n}" ::"r"(a), "r"(v)
-                 : "memory");
-}
 
 __device__ void tile8_visit(const G8 &g, int t, int tiles_x, int sweeps, int hlim, int round) {
     // excess and capacities have a ring too: flow that leaves the tile collects
@@ -225,10 +220,8 @@ __device__ void tile8_visit(const G8 &g, int t, int tiles_x, int sweeps, int hli
         // push half: heights fixed.  All loads first, the flows in registers,
         // then fire-and-forget atomics.
         int e = *(volatile int *)&se[ly + 1][lx + 1];
-        int hn[ND];
-        const bool on = e > 0 && hh <= hlim;
-        if (on) {
-            int cd[ND], f[ND];
+        if (e > 0 && hh <= hlim) {
+            int cd[ND], hn[ND];
 #pragma unroll
             for (int d = 0; d < ND; ++d) {
                 cd[d] = sc[d][ly + 1][lx + 1];
@@ -237,19 +230,16 @@ __device__ void tile8_visit(const G8 &g, int t, int tiles_x, int sweeps, int hli
             const int e_in = e;
 #pragma unroll
             for (int d = 0; d < ND; ++d) {
-                f[d] = hn[d] == hh - 1 ? min(e, cd[d]) : 0;
-                e -= f[d];
+                // zero or not: an add takes a cycle or two, a branch some twenty (with a
+                // test or a predicate per add 640x480 penalty 600 took 950 us, now 808)
+                const int f = hn[d] == hh - 1 ? min(e, cd[d]) : 0;
+                e -= f;
+                const int ny = ly + 1 + dyd(d), nx = lx + 1 + dxd(d);
+                atomicAdd(&sc[d][ly + 1][lx + 1], -f);
+                atomicAdd(&se[ny][nx], f);
+                atomicAdd(&sc[opp(d)][ny][nx], f);
             }
-            if (e != e_in) {
-#pragma unroll
-                for (int d = 0; d < ND; ++d) {
-                    const int ny = ly + 1 + dyd(d), nx = lx + 1 + dxd(d);
-                    if (f[d]) sc[d][ly + 1][lx + 1] = cd[d] - f[d];
-                    red_shared_if(&se[ny][nx], f[d]);
-                    red_shared_if(&sc[opp(d)][ny][nx], f[d]);
-                }
-                atomicSub(&se[ly + 1][lx + 1], e_in - e);
-            }
+            atomicAdd(&se[ly + 1][lx + 1], e - e_in);
         }
         if (threadIdx.x == 0) live[(s + 1) % 3] = 0;  // last read in sweep s - 2
         __syncthreads();
@@ -259,13 +249,11 @@ __device__ void tile8_visit(const G8 &g, int t, int tiles_x, int sweeps, int hli
             int m = INF_H;
 #pragma unroll
             for (int d = 0; d < ND; ++d) {
-                if (!on) hn[d] = sh[ly + 1 + dyd(d)][lx + 1 + dxd(d)];  // (others have them from the push half)
-                if (sc[d][ly + 1][lx + 1] > 0) m = min(m, hn[d]);
+                const int hn = sh[ly + 1 + dyd(d)][lx + 1 + dxd(d)];
+                m = min(m, sc[d][ly + 1][lx + 1] > 0 ? hn : INF_H);
             }
-            if (m >= hh) {
-                hh = m >= INF_H - 1 ? INF_H : m + 1;
-                sh[ly + 1][lx + 1] = hh;
-            }
+            if (m >= hh) hh = min(m, INF_H - 1) + 1;
+            sh[ly + 1][lx + 1] = hh;
         }
         // still active?  A flag per sweep, three in rotation (set before a
         // barrier, read after it, cleared two sweeps later)
@@ -672,7 +660,12 @@ __global__ void __launch_bounds__(256) k8_solve(G8 g, P8 prm) {
             break;
         }
         // ---- tile rounds: the due tiles, block-local sweeps ----
-        for (int p = 0; p < prm.rounds; ++p) {
+        // A graph that takes a fourth relabel moves its flow far: three times the
+        // rounds per relabel from there on (640x480 penalty 600 808 -> 771 us,
+        // 1920x1080 3086 -> 2596, 200x150 penalty 100 1303 -> 1109; twice 785,
+        // 2631, 1189; graphs of fewer relabels are unchanged).
+        const int rounds = outer > 2 ? 3 * prm.rounds : prm.rounds;
+        for (int p = 0; p < rounds; ++p) {
             // round_active[R % 3] counts this round's tiles and is read after the
             // round's barrier; the counter of round R + 1 was last read after
             // the barrier of round R - 2, which every block has passed

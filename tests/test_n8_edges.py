@@ -53,3 +53,26 @@ def test_sink_at_distance(dist, near):
         for k in DIRS:
             arrs[k][:, 110:] = rng.integers(0, 25, (h, 40))
     _check(dp, dn, 0, arrs)
+
+
+@pytest.mark.parametrize("rounds", [1, 2, 8])
+@pytest.mark.parametrize("w,h,penalty", [(70, 45, 60), (200, 150, 100)])
+def test_many_relabels(w, h, penalty, rounds):
+    """Sources on one side and sinks on the other: far flow, so that the solve
+    goes past its third relabel."""
+    import gcfg
+    import oracle as O
+    from gpu_util import dev
+
+    rng = np.random.default_rng(w + rounds)
+    dp = (rng.integers(0, 90, (h, w)) * (np.arange(w) < w // 3)).astype(np.int32)
+    dn = (rng.integers(0, 90, (h, w)) * (np.arange(w) > w // 2)).astype(np.int32)
+    gw = gcfg.GC_Init8(w, h, dev(dp), dev(dn), penalty)
+    gcfg.GC_SetSchedule8(gw, rounds, 3)
+    label = np.zeros((h, w), np.int32)
+    r = gcfg.GC_Optimize8(gw, label)
+    gcfg.GC_End8(gw)
+    o = O.solve8(dp, dn, penalty=penalty, arrays=None)
+    if rounds == 1:
+        assert r["global_relabels"] > 3
+    assert r["flow"] == o["flow"] and np.array_equal(label, o["smax"].astype(np.int32))
