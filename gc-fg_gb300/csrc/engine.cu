@@ -730,9 +730,14 @@ __device__ void reach_tile(const Batch &b, int t, bool round0, int tag_next, int
 // complement of S_max inside the image).  The expansion of tile_bfs without
 // levels.  round0: the neighbours' sets are not known yet, so the halo starts
 // from their sink-connected pixels; later rounds read their hfin rows, all
-// written by this pass (the sets only grow, so the rounds converge).
+// written by this pass (the sets only grow, so the rounds converge).  A set
+// that holds a pixel with excess settles the check for the image: it is open,
+// and its tiles' further visits end at once.  (A closure carried on to its end
+// floods all that the sinks can still be reached from, tile by tile, to no use.)
 __device__ void sink_reach_tile(const Batch &b, int t, bool round0, int tag_next, int slot_next) {
     const int lane = threadIdx.x & 31;
+    ImgState *ist = b.ist + __ldg(b.tile_img + t);
+    if (__any_sync(FULL, vload(&ist->done) || vload(&ist->open))) return;
     int nb[4];
     tile_nbs(b, t, nb);
     unsigned m[6];
@@ -755,6 +760,13 @@ __device__ void sink_reach_tile(const Batch &b, int t, bool round0, int tag_next
         const unsigned nw = ((Rl & ((S << 1) | lbit)) | (Rr & ((S >> 1) | rbit)) | (Ru & up) | (Rd & dn)) & ~S;
         if (!__any_sync(FULL, nw != 0)) break;
         S |= nw;
+    }
+    if (__any_sync(FULL, (S & m[5]) != 0)) {
+        if (lane == 0) {
+            *(volatile int *)&ist->open = 1;
+            *(volatile int *)&b.ctl->open_images = 1;
+        }
+        return;
     }
     b.hfin[(size_t)t * 32 + lane] = S;
     // a neighbour is queued when a pixel new in this tile's set has a facing
@@ -1195,17 +1207,10 @@ __device__ __noinline__ int closure_check(const Batch &b, const SolveParams &prm
     const int nt = batch_ntiles(b);
     for (int k = gtid; k < batch_nimg(b); k += nthreads) {
         const int i = batch_img(b, k);
-        if (!b.ist[i].done) {
-            b.ist[i].pos_excess = 0;
-            b.ist[i].active = 0;
-        }
+        if (!b.ist[i].done) b.ist[i].pos_excess = 0;
     }
-    if (gtid == 0) ctl->open_images = 0;
-    for (int k = gwarp; k < nt; k += nwarps) {
-        const int t = batch_tile(b, k);
-        if (vload(&b.ist[__ldg(b.tile_img + t)].done)) continue;  // warp-uniform
-        sink_reach_tile(b, t, true, G + 1, L_GR0 + ((G + 1) & 1));
-    }
+    for (int k = gwarp; k < nt; k += nwarps)
+        sink_reach_tile(b, batch_tile(b, k), true, G + 1, L_GR0 + ((G + 1) & 1));
     if (!grid_sync(b, 0)) return -1;
     ++G;
     for (int k = 1;; ++k) {
@@ -1221,18 +1226,7 @@ __device__ __noinline__ int closure_check(const Batch &b, const SolveParams &prm
         if (!grid_sync(b, 1u << slot)) return -1;
         ++G;
     }
-    // per image: any pixel with excess inside the closure (warp per tile), and
-    // the exact sum of positive excess (lane per tile)
-    for (int k = gwarp; k < nt; k += nwarps) {
-        const int t = batch_tile(b, k);
-        const int img = __ldg(b.tile_img + t);
-        if (vload(&b.ist[img].done)) continue;  // warp-uniform
-        const unsigned live = __ldcg(b.hfin + (size_t)t * 32 + lane) & mask_word(b, t, 5, lane);
-        if (__any_sync(FULL, live != 0) && lane == 0) {
-            b.ist[img].active = 1;
-            *(volatile int *)&ctl->open_images = 1;
-        }
-    }
+    // per image: the exact sum of positive excess (lane per tile)
     for (int kb = gtid - lane; kb < nt; kb += nthreads) {  // warp-uniform
         const int k = kb + lane;
         int img = -1;
@@ -1263,7 +1257,7 @@ __device__ __noinline__ int closure_check(const Batch &b, const SolveParams &prm
     }
     for (int k = gtid; k < batch_nimg(b); k += nthreads) {
         const int i = batch_img(b, k);
-        if (!b.ist[i].done && *(volatile unsigned long long *)&b.ist[i].active == 0) b.ist[i].done = 1;
+        if (!b.ist[i].done && !vload(&b.ist[i].open)) b.ist[i].done = 1;
     }
     if (!grid_sync(b, 0)) return -1;
     return 0;
@@ -1332,9 +1326,13 @@ __global__ void __launch_bounds__(NW * 32, solve_min_blocks<NW>()) k_solve(Batch
             if (!b.ist[i].done) {
                 b.ist[i].pos_excess = 0;
                 b.ist[i].active = 0;
+                b.ist[i].open = 0;  // for the next termination check, as open_images
             }
         }
-        if (gtid == 0) ctl->total_active = 0;
+        if (gtid == 0) {
+            ctl->total_active = 0;
+            ctl->open_images = 0;
+        }
         // round 0 visits every tile: with two or more per warp it is bound by
         // issue, and the short BFS with direct level stores is the cheaper one
         // (nt >= 2 * nwarps below)
