@@ -1205,28 +1205,10 @@ __device__ __noinline__ int closure_check(const Batch &b, const SolveParams &prm
     const int swarp = warp * gridDim.x + blockIdx.x;
     const int gtid = blockIdx.x * blockDim.x + threadIdx.x, nthreads = gridDim.x * blockDim.x;
     const int nt = batch_ntiles(b);
-    for (int k = gtid; k < batch_nimg(b); k += nthreads) {
-        const int i = batch_img(b, k);
-        if (!b.ist[i].done) b.ist[i].pos_excess = 0;
-    }
     for (int k = gwarp; k < nt; k += nwarps)
         sink_reach_tile(b, batch_tile(b, k), true, G + 1, L_GR0 + ((G + 1) & 1));
-    if (!grid_sync(b, 0)) return -1;
-    ++G;
-    for (int k = 1;; ++k) {
-        const int slot = L_GR0 + (G & 1);
-        const int n = vload(&ctl->size[slot]);
-        if (n == 0) break;
-        if (k > prm.max_rounds) {
-            if (gtid == 0) set_error(b, ERRC_GR_ROUNDS);
-            return -1;
-        }
-        for (int idx = swarp; idx < n; idx += nwarps)
-            sink_reach_tile(b, b.lists[(size_t)slot * b.list_cap + idx], false, G + 1, L_GR0 + ((G + 1) & 1));
-        if (!grid_sync(b, 1u << slot)) return -1;
-        ++G;
-    }
-    // per image: the exact sum of positive excess (lane per tile)
+    // beside round 0, per image: the exact sum of positive excess (lane per
+    // tile; cleared before the push rounds)
     for (int kb = gtid - lane; kb < nt; kb += nthreads) {  // warp-uniform
         const int k = kb + lane;
         int img = -1;
@@ -1250,6 +1232,20 @@ __device__ __noinline__ int closure_check(const Batch &b, const SolveParams &prm
         }
     }
     if (!grid_sync(b, 0)) return -1;
+    ++G;
+    for (int k = 1;; ++k) {
+        const int slot = L_GR0 + (G & 1);
+        const int n = vload(&ctl->size[slot]);
+        if (n == 0) break;
+        if (k > prm.max_rounds) {
+            if (gtid == 0) set_error(b, ERRC_GR_ROUNDS);
+            return -1;
+        }
+        for (int idx = swarp; idx < n; idx += nwarps)
+            sink_reach_tile(b, b.lists[(size_t)slot * b.list_cap + idx], false, G + 1, L_GR0 + ((G + 1) & 1));
+        if (!grid_sync(b, 1u << slot)) return -1;
+        ++G;
+    }
     if (gtid == 0) ctl->closure_checks++;
     if (vload(&ctl->open_images) == 0) {  // no image has an augmenting path left
         if (gtid == 0) ctl->closure_ends++;
@@ -1486,8 +1482,11 @@ __global__ void __launch_bounds__(NW * 32, solve_min_blocks<NW>()) k_solve(Batch
                 const int i = batch_img(b, k);
                 // under a height limit an image without active pixels may still have
                 // some beyond it: the termination check decides
-                if (hlim == INF_H - 1 && !b.ist[i].done && *(volatile unsigned long long *)&b.ist[i].active == 0)
+                if (b.ist[i].done) continue;
+                if (hlim == INF_H - 1 && *(volatile unsigned long long *)&b.ist[i].active == 0)
                     b.ist[i].done = 1;
+                else
+                    b.ist[i].pos_excess = 0;  // summed again by the termination check
             }
             if (total == 0) {
                 if (hlim == INF_H - 1) {
@@ -1495,6 +1494,7 @@ __global__ void __launch_bounds__(NW * 32, solve_min_blocks<NW>()) k_solve(Batch
                     break;
                 }
                 full = true;  // nothing to push within the limit
+                if (!grid_sync(b, 0)) return;  // (the sums are cleared)
                 continue;
             }
         }
