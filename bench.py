@@ -70,18 +70,19 @@ P99_TARGET_MS = 5.0
 UNIT = "Mpixel/s"
 
 # Algorithmic bytes per pixel per unit of work (int32 layout):
-#   global relabel: read 4 caps + excess (20 B), write height (4 B), once per
-#     pixel per global relabel; a tile that the BFS frontier visits again in
-#     a later round of the same relabel is overhead, not algorithmic bytes
+#   global relabel: read the residual and sign bits (6 bits), write the height
+#     (4 B), once per pixel per global relabel; a tile that the BFS visits again
+#     in the same relabel is overhead, not algorithmic bytes
 #   push tile visit (a tile active in a push round; push and local relabel
-#     fused): read 4 caps + excess + height (24 B), write the same (24 B)
-#   source reachability (cut): read 4 caps + excess (20 B), once per pixel at most
+#     fused): read 4 caps + excess + height (24 B), write the same (24 B; an
+#     upper bound: rows that did not change are not written)
+#   source reachability (cut): read the bits, write one, once per pixel at most
 #   sink reachability (the termination check after push rounds, which also
-#     gives S_max): the same 20 B, once per pixel per check
-#   count pass: read excess + height (8 B)
+#     gives S_max): the same, once per pixel per check
+#   count pass: two words per tile
 #   build: read RGB (3 B), write 4 caps + excess (20 B)
 #   extract: read height (4 B) + reach bit, write two label bytes (2 B)
-B_GR, B_PUSH, B_REACH, B_COUNT, B_BUILD, B_EXTRACT = 24, 48, 20, 8, 23, 6
+B_GR, B_PUSH, B_REACH, B_COUNT, B_BUILD, B_EXTRACT = 4.75, 48, 0.875, 12 / 1024, 23, 6
 
 # Bytes a solver phase really moves per tile visit in the tile-arena layout
 # (what DRAM counters see when nothing is served from L2):
@@ -566,7 +567,7 @@ def ncu_phase_traffic(kind, workload_name):
 
 
 def solve_phases(gcfg, stream, Ws, Hs, lams, d_rgb, d_scrib, offs, peak, workload_name, batched, bs=None):
-    """The solver's first exact global relabel and the push rounds after it,
+    """The solver's first global relabel (up to its height limit) and the push rounds after it,
     each as a launch of its own (gcfg_batch_phase_split), inside the NVTX
     range "phase_split".  A batch is split as one batch; the images of a
     per-image workload one at a time, as the plain solver runs them."""
@@ -616,10 +617,10 @@ def solve_phases(gcfg, stream, Ws, Hs, lams, d_rgb, d_scrib, offs, peak, workloa
                         launches=len(groups), tile_visits=tot["push_tiles"], sweeps=tot["push_sweeps"],
                         local_relabels=tot["push_local_relabels"], colour_phases=tot["push_phases"])
     return {"global_relabel": gr, "push": push, "grid_blocks": max(grid),
-            "how": "gcfg_batch_phase_split: launch 1 = initialisation + the first exact global relabel + its count "
-                   "pass, launch 2 = the push rounds that follow (until the next global relabel), CUDA events "
-                   "per launch; alg = int32 accounting (global relabel 24 B/px once + count 8 B/px; push 48 B/px "
-                   "per visited pixel); moved = what the phase reads and writes in this layout (relabel: mask "
+            "how": "gcfg_batch_phase_split: launch 1 = initialisation + the first global relabel (up to its height "
+                   "limit) + its count pass, launch 2 = the push rounds that follow (until the next global relabel), CUDA events "
+                   "per launch; alg = bit planes read and heights written by the relabel (4.75 B/px once); "
+                   "push 48 B/px per visited pixel; moved = what the phase reads and writes in this layout (relabel: mask "
                    "planes, halo lines, heights, border lines; push: the 24 KB tile in and out, halos, masks); "
                    "traffic = ncu dram__bytes_read.sum + dram__bytes_write.sum of the same launches"}
 

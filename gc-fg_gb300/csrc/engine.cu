@@ -3,8 +3,8 @@
 // Algorithm (exact max-flow on a 4-connected grid, the reference's model):
 //   excess e = dp - dn (+ inflow - outflow); heights = residual distance to
 //   the sink (sink-connected nodes, e < 0, have height 1); the solve ends
-//   when, after an exact global relabel, no node with e > 0 can reach the
-//   sink.  Cuts: S_max = nodes that cannot reach the sink (the reference's
+//   when no node with e > 0 can reach the sink, which a sink-side closure or
+//   an exact global relabel shows.  Cuts: S_max = nodes that cannot reach the sink (the reference's
 //   labels, GraphCutKernels.cu:228-351), S_min = nodes reachable from the
 //   source (from nodes with e > 0).
 //
@@ -1313,8 +1313,8 @@ __global__ void __launch_bounds__(NW * 32, solve_min_blocks<NW>()) k_solve(Batch
                 break;
             }
         }
-        // ------------------------ exact global relabel ------------------------
-        // (up to hlim: a height above it, or INF, means farther than hlim)
+        // ------------------------ global relabel ------------------------
+        // (exact without a limit; up to hlim: a height above it, or INF, means farther than hlim)
         timeline = prm.phase == 1 && blockIdx.x == 0 && threadIdx.x == 0;  // the phase-split diagnostic
         if (timeline) ctl->gr_time[0] = gtimer();
         for (int k = gtid; k < batch_nimg(b); k += nthreads) {

@@ -7,13 +7,13 @@
 // capacities are eight planes, cap[d * n + i] from pixel i toward direction
 // d (0 left, 1 right, 2 up, 3 down, 4 up-left, 5 up-right, 6 down-left,
 // 7 down-right).  One cooperative launch runs the whole solve:
-//   * exact global relabel: the distances to the sink-connected pixels
+//   * global relabel, exact but for the first (up to nine steps): the distances to the sink-connected pixels
 //     (excess < 0) over the residual edges, by rounds over 32x32 tiles with a
 //     bit-parallel BFS of each tile (gr8_tile);
 //   * count: pixels with excess that can still reach the sink; none left
 //     after an exact global relabel means the preflow is maximum (an exact
 //     termination test);
-//   * tile rounds: every 32x8 tile once per round, each visit a few
+//   * tile rounds: every 32x8 tile that is due once per round, each visit a few
 //     block-local push/relabel sweeps in shared memory (tile8_visit), the
 //     results added back as deltas;
 //   * cuts: S_max = pixels at height INF after the last exact global
@@ -764,12 +764,12 @@ struct gcfg_graph8 {
     Ctl8 *ctl = nullptr, *h_ctl = nullptr;
     cudaStream_t st = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev2 = nullptr;  // solve start, solve end, extract end
-    // schedule: 8 sweeps per visit; solve kernel at 12 / 8 / 6 / 4 tile rounds
-    // per global relabel: 640x480, penalty 600 957 / 963 / 978 / 1040 us, penalty
-    // 20 497 / 385 / 348 / 503, arrays 351 / 272 / 231 / 194, 1920x1080 penalty 600
-    // 3285 / 3344 / 3734 / 4182 (16 sweeps: 1102 / 991 / 980 / 1024, 579 / 471 /
-    // 428 / 397, 499 / 372 / 309 / 245, 3486 / 3517 / 3599 / 4039); 2 blocks per
-    // SM are as fast as 3
+    // schedule: 8 sweeps per visit; solve kernel at 12 / 8 / 6 tile rounds per
+    // global relabel (the same to the end): 640x480, penalty 600 801 / 808 / 840
+    // us, penalty 20 398 / 345 / 321, arrays 175 / 166 / 156, 1920x1080 penalty
+    // 600 2682 / 3086 / 3388; with three times as many from the fourth relabel on
+    // 8 rounds take 771, 347, 166 and 2596 (12 sweeps 825, 363, 178, 2636; 6 sweeps,
+    // twice as many, 802, 331, 163, 2895).  2 blocks per SM: 874, 361, 169, 3278
     int rounds = GCFG_N8_ROUNDS, max_outer = 100000, blocks_per_sm = 3, sweeps = GCFG_N8_SWEEPS;
 
     G8 g() const {

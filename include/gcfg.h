@@ -51,7 +51,7 @@ typedef struct {
     int32_t ref_energy;      /* the value GC_Optimize prints as "Final energy level"
                                 (GraphCut.cu:456-457): int32, border dp included */
     int32_t status;          /* gcfg_status of the solve */
-    int32_t global_relabels; /* exact global relabels run */
+    int32_t global_relabels; /* global relabels run (the first two up to a height limit) */
     int32_t gr_sweeps;       /* tile-frontier rounds inside global relabels */
     int32_t push_rounds;     /* checkerboard push phases (one colour each) */
     int32_t cut_sweeps;      /* tile-frontier rounds of the source-side reachability */
@@ -359,7 +359,7 @@ gcfg_status gcfg_batch_autotune(gcfg_batch *b, int n, const int *widths, const i
 /* Diagnostic: the batch's data term and build, then the solver's two main
  * phases as two separate launches of the persistent solver kernel, so that a
  * profiler (or the events below) sees each on its own: launch 1 = the first
- * exact global relabel with its count pass (the reference's InitGlobalRelabel
+ * global relabel (up to the height limit) with its count pass (the reference's InitGlobalRelabel
  * + GlobalRelabel, GraphCutKernels.cu:757-875), launch 2 = the push rounds
  * that follow it (WavePush + Relabel, GraphCutKernels.cu:433-724).  The solve
  * is left unfinished (no cut); run the batch again for results.  Current
@@ -368,7 +368,7 @@ typedef struct {
     float ms_relabel;             /* device time of launch 1 */
     float ms_push;                /* device time of launch 2 (0 when nothing was active) */
     int64_t relabel_tiles;        /* global-relabel tile visits of launch 1 */
-    int64_t active_pixels;        /* pixels with excess and finite height after the relabel */
+    int64_t active_pixels;        /* pixels with excess and a height within the limit after the relabel */
     int64_t push_tiles;           /* push tile visits of launch 2 */
     int64_t push_sweeps;          /* push/relabel sweeps of those visits */
     int64_t push_local_relabels;  /* exact local relabels of those visits */
@@ -378,8 +378,9 @@ typedef struct {
     int32_t grid_blocks;          /* blocks of each launch */
     /* timeline of launch 1's global relabel (device clock, microseconds):
      * round 0 (every tile, halos from the neighbours' sink pixels), the pull
-     * check that picks the first frontier, then frontier round k with
-     * relabel_front_tiles[k] tiles, for k < min(relabel_rounds, 32) */
+     * check, then round k with relabel_front_tiles[k] tiles, for
+     * k < min(relabel_rounds, 32); under the height limit the one round is the
+     * refining visits that follow each tile's check at once */
     float relabel_round0_us, relabel_pull_us;
     float relabel_front_us[32];
     int32_t relabel_front_tiles[32];
