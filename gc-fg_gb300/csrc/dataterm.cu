@@ -442,6 +442,7 @@ __global__ void __launch_bounds__(1024) k_tlut_b(const int *__restrict__ ilist, 
                                                  int2 *__restrict__ tl_lut,
                                                  double *raw_dp, double *raw_dn) {
     __shared__ long long part[2][32];
+    cudaGridDependencySynchronize();
     const int im = ilist ? ilist[blockIdx.x] : blockIdx.x;
     if (threadIdx.x == blockDim.x - 1) img_params(img, ist, im);
     const int *hf = hist + (size_t)im * 2 * NBINS;
@@ -685,6 +686,7 @@ __global__ void __launch_bounds__(WARPS * 32, 32 / WARPS) k_build_img_b(Batch b,
     constexpr int STRIP = TILE_H / WARPS;
     __shared__ uint32_t msk[6][TILE_H];  // mask planes of the tile, stored coalesced below
     __shared__ unsigned long long wsum[3][WARPS];
+    cudaGridDependencySynchronize();
     const int t = batch_tile(b, blockIdx.x);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int im = __ldg(b.tile_img + t);
@@ -807,8 +809,8 @@ gcfg_status dt_tables(const DtArgs &a, cudaStream_t st) {
                                                                                 a.chunk, a.hist, a.ist));
     if (a.scrib)
         GCFG_LAUNCH(GCFG_PK_TLUT, st,
-                    k_tlut_b<<<a.n_img, 1024, 0, st>>>(a.ilist, a.hist, a.img, a.ist, a.tl_lut, a.raw_dp,
-                                                       a.raw_dn));
+                    launch_behind(k_tlut_b, a.n_img, 1024, st, a.ilist, a.hist, a.img, a.ist, a.tl_lut, a.raw_dp,
+                                  a.raw_dn));
     else
         GCFG_LAUNCH(GCFG_PK_TLUT, st,
                     k_img_params<<<div_up(a.n_img, 128), 128, 0, st>>>(a.ilist, a.img, a.n_img, a.ist));
@@ -819,9 +821,9 @@ gcfg_status dt_tables(const DtArgs &a, cudaStream_t st) {
 gcfg_status dt_build(const Batch &b, const DtArgs &a, cudaStream_t st) {
     const int tiles = batch_ntiles(b);
     if (tiles <= BUILD_SMALL_TILES)
-        GCFG_LAUNCH(GCFG_PK_BUILD, st, k_build_img_b<8><<<tiles, 256, 0, st>>>(b, a.rgb, a.tl_lut));
+        GCFG_LAUNCH(GCFG_PK_BUILD, st, launch_behind(k_build_img_b<8>, tiles, 256, st, b, a.rgb, a.tl_lut));
     else
-        GCFG_LAUNCH(GCFG_PK_BUILD, st, k_build_img_b<4><<<tiles, 128, 0, st>>>(b, a.rgb, a.tl_lut));
+        GCFG_LAUNCH(GCFG_PK_BUILD, st, launch_behind(k_build_img_b<4>, tiles, 128, st, b, a.rgb, a.tl_lut));
     GCFG_CK(cudaGetLastError());
     return GCFG_OK;
 }

@@ -1669,6 +1669,7 @@ __device__ __forceinline__ uint4 spread16(uint32_t bits) {
 __global__ void __launch_bounds__(256) k_extract_rows(Batch b, const int2 *__restrict__ chunk_map, int chunk,
                                                       uint8_t *smin, uint8_t *smax) {
     __shared__ long long s_row0;
+    cudaGridDependencySynchronize();
     const int2 cm = __ldg(chunk_map + blockIdx.x);
     const int W = __ldg(&b.img[cm.x].W), H = __ldg(&b.img[cm.x].H);
     const int tile0 = __ldg(&b.img[cm.x].tile0), tiles_x = __ldg(&b.img[cm.x].tiles_x);
@@ -1815,7 +1816,7 @@ gcfg_status launch_extract_rows(const Batch &b, const int2 *chunk_map, long long
         // the windows need one alignment for both arrays: the tile-major kernel instead
         return launch_extract(b, smin, smax, nullptr, st);
     }
-    GCFG_LAUNCH(GCFG_PK_EXTRACT, st, k_extract_rows<<<(unsigned)n_chunks, 256, 0, st>>>(b, chunk_map, chunk, smin, smax));
+    GCFG_LAUNCH(GCFG_PK_EXTRACT, st, launch_behind(k_extract_rows, (unsigned)n_chunks, 256, st, b, chunk_map, chunk, smin, smax));
     GCFG_CK(cudaGetLastError());
     return GCFG_OK;
 }

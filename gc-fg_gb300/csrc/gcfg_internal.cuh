@@ -61,6 +61,23 @@ void prof_begin(cudaStream_t st);
 void prof_end(int kind, cudaStream_t st);
 
 // Launch a kernel, counting it and (when profiling) timing it with events.
+// Launch of a kernel that follows another kernel in the stream and begins with
+// cudaGridDependencySynchronize(): it is set up while the last blocks of that
+// one run, and waits there until all of it, results included, is done.
+template <typename... P, typename... A>
+inline cudaError_t launch_behind(void (*k)(P...), unsigned blocks, unsigned threads, cudaStream_t st, A... args) {
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c = {};
+    c.gridDim = dim3(blocks);
+    c.blockDim = dim3(threads);
+    c.stream = st;
+    c.attrs = &at;
+    c.numAttrs = 1;
+    return cudaLaunchKernelEx(&c, k, P(args)...);
+}
+
 #define GCFG_LAUNCH(kind, st, ...)                      \
     do {                                                \
         ::gcfg::prof_begin(st);                         \
