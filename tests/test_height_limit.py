@@ -45,3 +45,29 @@ def test_far_sinks_behind_weak_edges(seed):
     kw = {k: (rng.integers(0, 25, (H, W)) * (rng.random((H, W)) < 0.85)).astype(np.int32)
           for k in ("up", "down", "left", "right")}
     _check(dp, dn, **kw)
+
+
+@pytest.mark.parametrize("seed", range(3))
+def test_easy_and_hard_images_in_one_solve(seed):
+    """Images that end at their first termination check beside images that
+    need several: each image's check is its own."""
+    import gcfg
+    import oracle as O
+    from gpu_util import dev
+
+    rng = np.random.default_rng(seed)
+    ims = [(int(rng.integers(20, 200)), int(rng.integers(20, 200)), lam)
+           for lam in (1.0, 20000.0, 50.0, 2000.0, 10.0, 100000.0, 200.0, 5000.0)]
+    data = [O.generate(3, w, h, seed * 100 + i) for i, (w, h, _) in enumerate(ims)]
+    rgb, scrib = (dev(np.concatenate([d[k].reshape(-1) for d in data])) for k in (0, 1))
+    smin, smax = torch.zeros_like(scrib), torch.zeros_like(scrib)
+    bs = gcfg.BatchSolver(len(ims), scrib.numel())
+    flows, _ = bs.run([w for w, _, _ in ims], [h for _, h, _ in ims], [lam for *_, lam in ims], rgb, scrib, smin, smax)
+    bs.close()
+    a, b, off = smin.cpu().numpy(), smax.cpu().numpy(), 0
+    for (w, h, lam), (im, sc), flow in zip(ims, data, flows):
+        o = O.segment(im, sc, lam)
+        assert flow == o["flow"]
+        assert np.array_equal(a[off:off + w * h].reshape(h, w), o["smin"])
+        assert np.array_equal(b[off:off + w * h].reshape(h, w), o["smax"])
+        off += w * h
