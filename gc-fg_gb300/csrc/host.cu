@@ -116,7 +116,7 @@ struct Engine {
     std::vector<GraphEntry> graphs;
     cudaStream_t cap_st = nullptr;
     long long graph_kernels = 0, graph_replays = 0, graph_captures = 0, graph_clock = 0;
-    long long alloc_gen = 0;  // bumped whenever a buffer is reallocated
+    long long alloc_gen = 0;  // bumped whenever a buffer is reallocated (see reserve)
 
     // Host entry points of many images: groups of consecutive images are
     // uploaded on cp_st while earlier groups already compute on st.
@@ -308,13 +308,16 @@ struct Engine {
         carve_host(nullptr);
     }
 
-    std::vector<const void *> buffers() const { return {slab, h_slab, d_rgb, d_scrib, d_smin, d_smax}; }
-
-    // Grow the buffers; any reallocation invalidates the captured graphs.
+    // Grow the buffers.  alloc_gen goes up whenever an address that a captured
+    // graph may hold has changed.  The arrays carved out of a slab move with
+    // its capacities, even where the new slab has the old one's address, so a
+    // new slab always counts (reserve_); the staging buffers are one array
+    // each, and count if their address changed.
     gcfg_status reserve(int imgs, int tiles, long long px, bool dataterm, bool staging) {
-        const std::vector<const void *> before = buffers();
+        auto staged = [&] { return std::vector<const void *>{d_rgb, d_scrib, d_smin, d_smax}; };
+        const std::vector<const void *> before = staged();
         const gcfg_status rc = reserve_(imgs, tiles, px, dataterm, staging);
-        if (buffers() != before) ++alloc_gen;
+        if (staged() != before) ++alloc_gen;
         return rc;
     }
 
@@ -322,6 +325,7 @@ struct Engine {
         const size_t chunks = (size_t)max_chunks(imgs, px);
         if (!slab || (size_t)imgs > cap_imgs || chunks > cap_chunks || (size_t)tiles > cap_tiles ||
             (dataterm && !cap_dt)) {
+            ++alloc_gen;
             cudaFree(slab);
             slab = nullptr;
             lay_w.clear();  // nothing is laid out any more
@@ -340,6 +344,7 @@ struct Engine {
             carve_device(slab);
         }
         if (!h_slab || h_imgs != cap_imgs || h_chunks != cap_chunks || h_tiles != cap_tiles) {
+            ++alloc_gen;
             free_host();
             h_imgs = cap_imgs;
             h_chunks = cap_chunks;
