@@ -322,6 +322,9 @@ __device__ unsigned tile_bfs_gr(unsigned Rl, unsigned Rr, unsigned Ru, unsigned 
     // write the levels of the pixels reached in this segment (and, at the end,
     // INF for the pixels never reached)
     auto flush = [&](bool final) {
+        // the levels are stored by four lanes and read by all; the loop may
+        // have ended (at the limit) with the store of the last ones
+        __syncwarp();
 #pragma unroll
         for (int k = 0; k < GR_NPL; ++k) sc.pl[k][lane] = P[k];
         sc.reached[lane] = S;
