@@ -437,7 +437,7 @@ __global__ void __launch_bounds__(256, 8) k_hist_sigma_b(const uint8_t *__restri
 
 // Per-bin t-link tables (one block per image, double precision), and the
 // image's n-link constants by the block's last thread.
-__global__ void __launch_bounds__(1024) k_tlut_b(const int *__restrict__ ilist, const int *__restrict__ hist,
+__global__ void __launch_bounds__(1024) k_tlut_b(const int *__restrict__ ilist, const int *hist,
                                                  const ImgDesc *__restrict__ img, ImgState *ist,
                                                  int2 *__restrict__ tl_lut,
                                                  double *raw_dp, double *raw_dn) {
@@ -593,6 +593,9 @@ __device__ __forceinline__ void build_strip(const BuildTile &g, const NlinkParam
         return use ? w : 0;
     };
     auto inside = [&](int px, int y) { return px >= 1 && px <= W - 2 && y >= 1 && y <= H - 2; };
+    // the arena is no table: the next rows' gathers may go ahead of its stores
+    int4 *__restrict__ cap = g.cap;
+    int *__restrict__ exc = g.exc;
     const bool col_in = x >= 1 && x <= W - 2, cols_in = x >= 1 && x <= W - 3;  // the lane's and the next column
 
     constexpr int AHEAD = 3;  // rows of words in flight
@@ -643,7 +646,7 @@ __device__ __forceinline__ void build_strip(const BuildTile &g, const NlinkParam
         k.w = wd;
         int e = 0;
         if (INNER || (x < W && y < H)) {
-            const int2 v = __ldg(g.lut + color_binw(c));
+            const int2 v = g.lut[color_binw(c)];
             const bool counted = INNER ? r * w32 < left : (long long)x + (long long)y * w32 < (long long)W * H;
             if (counted) rinit += (unsigned)max(v.x, 0);
             if (INNER || inside(x, y)) {
@@ -651,8 +654,8 @@ __device__ __forceinline__ void build_strip(const BuildTile &g, const NlinkParam
                 idp += (unsigned)v.x;
             }
         }
-        g.cap[r * 32] = k;
-        g.exc[r * 32] = e;
+        cap[r * 32] = k;
+        exc[r * 32] = e;
         pos += (unsigned)max(e, 0);
         // of the six mask planes, the left one is the right one moved by a
         // column, the upper one the lower one of the row before
@@ -682,7 +685,7 @@ __device__ __forceinline__ void build_strip(const BuildTile &g, const NlinkParam
 constexpr int BUILD_SMALL_TILES = 1024;
 template <int WARPS>
 __global__ void __launch_bounds__(WARPS * 32, 32 / WARPS) k_build_img_b(Batch b, const uint8_t *__restrict__ rgb,
-                                                                   const int2 *__restrict__ tl_lut) {
+                                                                   const int2 *tl_lut) {
     constexpr int STRIP = TILE_H / WARPS;
     __shared__ uint32_t msk[6][TILE_H];  // mask planes of the tile, stored coalesced below
     __shared__ unsigned long long wsum[3][WARPS];

@@ -1699,11 +1699,12 @@ __global__ void __launch_bounds__(256) k_extract_rows(Batch b, const int2 *__res
             const int len = min(e - pos, W - x);
             const int sh = x & 31, r = y & 31;
             const size_t t = (size_t)tile0 + (size_t)(y >> 5) * tiles_x + (x >> 5);
-            const unsigned f0 = __ldg(b.hfin + t * 32 + r), r0 = __ldg(b.reach + t * 32 + r);
+            // (plain loads: the solver may still run when this kernel is set up)
+            const unsigned f0 = b.hfin[t * 32 + r], r0 = b.reach[t * 32 + r];
             unsigned f1 = 0, r1 = 0;
             if (sh + len > 32) {  // the segment reaches into the next tile of the row
-                f1 = __ldg(b.hfin + (t + 1) * 32 + r);
-                r1 = __ldg(b.reach + (t + 1) * 32 + r);
+                f1 = b.hfin[(t + 1) * 32 + r];
+                r1 = b.reach[(t + 1) * 32 + r];
             }
             const unsigned keep = len >= 32 ? 0xFFFFFFFFu : (1u << len) - 1u;
             // interior pixels: not on row 0 or H - 1, not at x = 0 or W - 1

@@ -56,14 +56,16 @@ extern std::atomic<long long> g_launches;
 
 constexpr int PK_COUNT_KINDS = GCFG_PK_NKINDS;
 bool prof_on();
-bool prof_on();
 void prof_begin(cudaStream_t st);
 void prof_end(int kind, cudaStream_t st);
 
-// Launch a kernel, counting it and (when profiling) timing it with events.
 // Launch of a kernel that follows another kernel in the stream and begins with
 // cudaGridDependencySynchronize(): it is set up while the last blocks of that
-// one run, and waits there until all of it, results included, is done.
+// one run, and waits there until all of it, results included, is done.  Such
+// a kernel exists before its producer has ended, so it reads what the producer
+// writes by plain loads, behind that call: not by __ldg nor through a const
+// __restrict__ pointer, which promise data that is constant for the kernel's
+// whole life.
 template <typename... P, typename... A>
 inline cudaError_t launch_behind(void (*k)(P...), unsigned blocks, unsigned threads, cudaStream_t st, A... args) {
     cudaLaunchAttribute at;
@@ -78,6 +80,7 @@ inline cudaError_t launch_behind(void (*k)(P...), unsigned blocks, unsigned thre
     return cudaLaunchKernelEx(&c, k, P(args)...);
 }
 
+// Launch a kernel, counting it and (when profiling) timing it with events.
 #define GCFG_LAUNCH(kind, st, ...)                      \
     do {                                                \
         ::gcfg::prof_begin(st);                         \
