@@ -1797,6 +1797,7 @@ gcfg_status launch_solve(const Batch &b, const SolveParams &prm, int n_tiles, cu
     const SolveKernel k = solve_kernel(warps);
     Batch bb = b;
     SolveParams pp = prm;
+    if (pp.max_sweeps > MAX_SWEEPS) pp.max_sweeps = MAX_SWEEPS;
     void *args[] = {&bb, &pp};
     prof_begin(st);
     const cudaError_t e = cudaLaunchCooperativeKernel(k.fn, dim3(grid), dim3(warps * 32), args, k.smem, st);

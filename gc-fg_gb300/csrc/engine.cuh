@@ -146,6 +146,12 @@ struct SolveParams {
                        // 4, 8, 16 or 32; 0: by the solve's size (solve_warps)
 };
 
+// More sweeps per visit than this are taken as this many (launch_solve): the
+// settings accept any count, the solver doubles it in long solves, and a
+// visit, which ends by itself when its tile has nothing left to push, is to
+// have a bound in time (a sweep takes about 1 us).
+constexpr int MAX_SWEEPS = 1 << 16;
+
 // Default solver settings of every entry point (before any tuning): 2 push
 // rounds per global relabel, 16 sweeps per tile visit, an exact local relabel
 // every 4 sweeps.  Measured on single images from 256x256 to 4096x4096 and on

@@ -172,6 +172,11 @@ constexpr int T8W = 32, T8H = 8;
 #ifndef GCFG_N8_SWEEPS
 #define GCFG_N8_SWEEPS 8    // sweeps per tile visit
 #endif
+// More rounds than this between relabels are taken as this many: the setting
+// accepts any count, a long solve takes three times as many, and pixels whose
+// excess cannot reach a sink keep their tiles due, a few levels higher per
+// round, until a relabel finds them cut off.
+constexpr int MAX_ROUNDS8 = 1 << 12;
 
 __device__ void tile8_visit(const G8 &g, int t, int tiles_x, int sweeps, int hlim, int round) {
     // excess and capacities have a ring too: flow that leaves the tile collects
@@ -910,7 +915,7 @@ gcfg_status gcfg_optimize8(gcfg_graph8 *g, int32_t *host_label, gcfg_result *res
     // open, flow has to travel, and the limited iteration is in the way
     // (640x480 / 1920x1080, us without -> with: arrays 272 -> 177, 602 -> 393;
     // penalty 600 963 -> 995, 3344 -> 4285).
-    P8 prm{g->max_outer, g->rounds, g->sweeps, g->varying ? 9 : 0};
+    P8 prm{g->max_outer, g->rounds < MAX_ROUNDS8 ? g->rounds : MAX_ROUNDS8, g->sweeps, g->varying ? 9 : 0};
     void *args[] = {&gg, &prm};
     GCFG_CK(cudaEventRecord(g->ev0, g->st));
     GCFG_CK(cudaLaunchCooperativeKernel((const void *)k8_solve, dim3((unsigned)grid), dim3(256), args, 0, g->st));
