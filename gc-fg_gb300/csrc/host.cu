@@ -722,11 +722,7 @@ gcfg_status gcfg_optimize(gcfg_graph *g, int32_t *host_label, gcfg_result *res) 
     GCFG_CK(cudaEventRecord(e.ev0, e.st));
     GCFG_TRY(e.solve());
     GCFG_CK(cudaEventRecord(e.ev1, e.st));
-    if (host_label) {
-        GCFG_TRY(launch_extract(e.batch(), nullptr, nullptr, e.d_label, e.st));
-        GCFG_CK(cudaMemcpyAsync(host_label, e.d_label, (size_t)g->W * g->H * sizeof(int32_t), cudaMemcpyDeviceToHost,
-                                e.st));
-    }
+    if (host_label) GCFG_TRY(launch_extract(e.batch(), nullptr, nullptr, e.d_label, e.st));
     GCFG_TRY(e.fetch());
     // the graph is consumed in place, as in the reference: re-solving needs
     // gcfg_set_graph again (GraphCut.cu:385-534 leaves the residual graph)
@@ -735,7 +731,14 @@ gcfg_status gcfg_optimize(gcfg_graph *g, int32_t *host_label, gcfg_result *res) 
     float ms = 0.f;
     cudaEventElapsedTime(&ms, e.ev0, e.ev1);
     if (res) e.result(0, res, ms);
-    return e.status();
+    GCFG_TRY(e.status());
+    // the labels last: the caller's array keeps its contents when a solve fails
+    if (host_label) {
+        GCFG_CK(cudaMemcpyAsync(host_label, e.d_label, (size_t)g->W * g->H * sizeof(int32_t), cudaMemcpyDeviceToHost,
+                                e.st));
+        GCFG_CK(cudaStreamSynchronize(e.st));
+    }
+    return GCFG_OK;
 }
 
 gcfg_status gcfg_get_cuts(gcfg_graph *g, uint8_t *d_smin, uint8_t *d_smax) {

@@ -95,8 +95,8 @@ gcfg_status gcfg_set_graph(gcfg_graph *g);
 /* GC_Optimize: solve to the exact max flow.  If host_label != NULL it
  * receives W*H int32 labels: 1 = source side of the maximal source set
  * (pixels that cannot reach the sink), 0 = sink side and the 1-pixel border,
- * exactly like the reference's output (GraphCut.cu:507-529).  res may be
- * NULL. */
+ * exactly like the reference's output (GraphCut.cu:507-529); a solve that
+ * fails leaves it as it was.  res may be NULL. */
 gcfg_status gcfg_optimize(gcfg_graph *g, int32_t *host_label, gcfg_result *res);
 /* After gcfg_optimize: both canonical cuts into device buffers (W*H bytes
  * each, either may be NULL): smin = pixels reachable from the source in the
@@ -140,7 +140,9 @@ gcfg_status gcfg_set_graph8(gcfg_graph8 *g);
  * solve kernel), gr_sweeps (tile rounds of the global relabels),
  * gr_tiles (their 32x32 tile visits), push_rounds (tile rounds), push_tiles
  * (32x8 tile visits that had work) and cut_sweeps (tile rounds of the
- * source-side closure); the other fields are 0. */
+ * source-side closure); the other fields are 0.  Unlike gcfg_optimize it
+ * copies the labels before it knows the status: after a failed solve
+ * host_label is undefined. */
 gcfg_status gcfg_optimize8(gcfg_graph8 *g, int32_t *host_label, gcfg_result *res);
 gcfg_status gcfg_get_cuts8(gcfg_graph8 *g, uint8_t *d_smin, uint8_t *d_smax);
 gcfg_status gcfg_end8(gcfg_graph8 *g);
