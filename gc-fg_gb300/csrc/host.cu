@@ -622,6 +622,7 @@ struct gcfg_graph {
     bool varying = false;
     bool built = false;
     bool solved = false;
+    bool fresh = false;  // gcfg_init's upload may still be queued on its stream
 };
 
 struct gcfg_segmenter {
@@ -671,6 +672,7 @@ gcfg_status gcfg_set_graph(gcfg_graph *g) {
     GCFG_TRY(launch_build_arrays(e.batch(), g->dp, g->dn, g->penalty, g->varying ? g->up : nullptr, g->down,
                                  g->left, g->right, e.st));
     GCFG_TRY(e.fetch());
+    g->fresh = false;
     if (e.h_ctl->err) return GCFG_ERR_INVALID;  // capacities out of range
     g->built = true;
     g->solved = false;
@@ -689,6 +691,7 @@ gcfg_status gcfg_init(int w, int h, const int32_t *dp, const int32_t *dn, int32_
     g->e.want_label = (size_t)w * h;
     gcfg_status rc = g->e.init();
     if (rc == GCFG_OK) rc = g->e.layout(1, &w, &h, nullptr, false, false);
+    g->fresh = true;
     if (rc == GCFG_OK && dp) {
         gcfg_set_dataterms(g, dp, dn);
         if (up) rc = gcfg_set_edges(g, up, down, left, right);
@@ -704,6 +707,13 @@ gcfg_status gcfg_init(int w, int h, const int32_t *dp, const int32_t *dn, int32_
 
 gcfg_status gcfg_set_stream(gcfg_graph *g, void *stream) {
     if (!g) return GCFG_ERR_INVALID;
+    // A handle made without terms has its layout upload and the clearing of its
+    // control block queued on the stream it was made on: nothing of the new
+    // stream may come before them (every other call ends synchronised).
+    if (g->fresh && (cudaStream_t)stream != g->e.st) {
+        GCFG_CK(cudaStreamSynchronize(g->e.st));
+        g->fresh = false;
+    }
     g->e.st = (cudaStream_t)stream;
     return GCFG_OK;
 }
