@@ -54,3 +54,56 @@ def test_captured_graph_after_the_buffers_grew():
         b.run(bs)
     assert bs.graph_info()["captures"] == 3
     bs.close()
+
+
+def test_the_same_layout_after_another_one():
+    few, many = _few_and_many()
+    other = _Batch([(150, 90), (65, 200), (33, 40)], 7200)  # the sizes of `few`, other images
+    weak = _Batch([(150, 90), (65, 200), (33, 40)], 7000, lam=3.0)  # and other lambdas
+    bs = gcfg.BatchSolver(64, max(few.scrib.size, many.scrib.size))
+    for b in (few, few, other, many, few, weak, weak, other, many, many, few):
+        b.run(bs)
+    bs.close()
+
+
+def test_stream_changed_between_runs_of_one_layout():
+    few, _ = _few_and_many()
+    other = _Batch([(150, 90), (65, 200), (33, 40)], 7200)
+    bs = gcfg.BatchSolver(len(few.W), few.scrib.size)
+    torch.cuda.synchronize()
+    for stream in (None, torch.cuda.Stream(), torch.cuda.Stream(), None):
+        if stream is not None:
+            stream.wait_stream(torch.cuda.current_stream())
+        bs.set_stream(stream if stream is not None else torch.cuda.current_stream())
+        with torch.cuda.stream(stream):
+            other.run(bs)
+            few.run(bs)
+    bs.close()
+
+
+@pytest.mark.parametrize("graph", [False, True])
+def test_growth_while_a_batch_is_in_flight(graph):
+    """The second set of host tables and staging buffers is made, and every
+    device array moves, while the first batch is on its way."""
+    few, many = _few_and_many()
+    big = _Batch([(400, 300), (90, 500)], 7300)
+    bs = gcfg.BatchSolver(len(few.W), few.scrib.size)
+    bs.set_graph(graph)
+    pinned = {id(b): [torch.from_numpy(a).pin_memory().numpy() for a in (b.rgb, b.scrib)] for b in (few, many, big)}
+
+    def submit(b):
+        out = [torch.full((b.scrib.size,), 7, dtype=torch.uint8).pin_memory().numpy() for _ in range(2)]
+        return b, out, bs.submit_host(b.W, b.H, b.lam, *pinned[id(b)], *out)
+
+    def collect(flight):
+        b, out, ticket = flight
+        b.check(bs.wait(ticket)[0], out)
+
+    flight = submit(few)
+    for b in (many, big, few, few, many, few, big, big):
+        nxt = submit(b)
+        collect(flight)
+        flight = nxt
+    collect(flight)
+    few.run(bs)
+    bs.close()
