@@ -106,8 +106,11 @@ gcfg_status gcfg_get_cuts(gcfg_graph *g, uint8_t *d_smin, uint8_t *d_smax);
 gcfg_status gcfg_end(gcfg_graph *g);
 /* Stream used by every later call on this graph (void* = cudaStream_t). */
 gcfg_status gcfg_set_stream(gcfg_graph *g, void *stream);
-/* Checkerboard push rounds between global relabels, and push/relabel sweeps
- * per tile visit (solver schedule; does not change the result). */
+/* Checkerboard push rounds between global relabels (default 2), and
+ * push/relabel sweeps per tile visit (default 16; a solve that goes on past its
+ * first iteration without a height limit takes twice as many from there on;
+ * counts above 65,536 are taken as 65,536).  Solver schedule; does not change
+ * the result. */
 gcfg_status gcfg_set_schedule(gcfg_graph *g, int push_rounds_per_gr, int max_tile_sweeps);
 
 /* ---------------- graph API with the 8-neighbourhood ---------------- */
@@ -151,6 +154,7 @@ gcfg_status gcfg_set_stream8(gcfg_graph8 *g, void *stream);
  * three times as many; every 32x8 tile that is due is
  * visited once per round, with up to 8 block-local push/relabel sweeps) and
  * blocks of the cooperative launch per SM (default 3; 0 = as many as fit);
+ * rounds above 4,096 are taken as 4,096;
  * the solver schedule only, results do not depend on it. */
 gcfg_status gcfg_set_schedule8(gcfg_graph8 *g, int rounds_per_gr, int blocks_per_sm);
 
@@ -282,7 +286,8 @@ typedef struct gcfg_batch gcfg_batch;
 gcfg_status gcfg_batch_create(int max_images, int64_t max_pixels, gcfg_batch **out);
 gcfg_status gcfg_batch_set_stream(gcfg_batch *b, void *stream);
 /* Solver schedule: push rounds between global relabels, sweeps per tile
- * visit, sweeps between exact local relabels (does not change results). */
+ * visit (both as in gcfg_set_schedule), sweeps between exact local relabels
+ * (default 4).  Does not change results. */
 gcfg_status gcfg_batch_set_params(gcfg_batch *b, int push_rounds_per_gr, int max_tile_sweeps,
                                   int sweeps_per_local_relabel);
 /* Device-resident batch.  d_smin/d_smax (packed, may be NULL) receive the
@@ -331,7 +336,7 @@ gcfg_status gcfg_batch_graph_info(gcfg_batch *b, int *active, int64_t *captures,
  * the width of the bit-plane tile BFS (one 32-bit mask per row). */
 typedef struct {
     int32_t push_rounds_per_gr;       /* checkerboard push rounds between global relabels */
-    int32_t max_tile_sweeps;          /* push/relabel sweeps per tile visit */
+    int32_t max_tile_sweeps;          /* push/relabel sweeps per tile visit (gcfg_set_schedule) */
     int32_t sweeps_per_local_relabel; /* sweeps between exact local (tile BFS) relabels */
     int32_t blocks_per_sm;            /* persistent solver blocks per SM (for one image: blocks per image / SMs) */
     float ms_default, ms_best;        /* device time of one run before / after tuning */
