@@ -28,11 +28,6 @@ __device__ __forceinline__ int color_bin3(const uint8_t *__restrict__ p) {
     return ((p[0] >> 4) << 8) | ((p[1] >> 4) << 4) | (p[2] >> 4);
 }
 
-__device__ __forceinline__ int diff2p(const uint8_t *__restrict__ a, const uint8_t *__restrict__ b) {
-    const int d0 = (int)a[0] - b[0], d1 = (int)a[1] - b[1], d2 = (int)a[2] - b[2];
-    return d0 * d0 + d1 * d1 + d2 * d2;
-}
-
 // Colour of a pixel as one word: r | g << 8 | b << 16.
 __device__ __forceinline__ uint32_t pack_rgb(const uint8_t *__restrict__ p) {
     return (uint32_t)__ldg(p) | ((uint32_t)__ldg(p + 1) << 8) | ((uint32_t)__ldg(p + 2) << 16);

@@ -1389,9 +1389,9 @@ __global__ void __launch_bounds__(NW * 32, solve_min_blocks<NW>()) k_solve(Batch
                     stat_add(st, ST_CYC_GR, cyc);
                     stat_add(st, ST_GR_TILES, 1ull);
                     if (prm.phase == 1) {  // the phase-split diagnostic only: shown as frontier round 0
-                        atomicAdd(&ctl->gr_front[0], 1);
-                        atomicMax(&ctl->gr_front_end[0], gtimer());
-                        atomicMax(&ctl->gr_front_maxcyc[0], cyc);
+                        atomicAdd(&ctl->gr_front, 1);
+                        atomicMax(&ctl->gr_front_end, gtimer());
+                        atomicMax(&ctl->gr_front_maxcyc, cyc);
                     }
                 }
             }
@@ -1425,7 +1425,7 @@ __global__ void __launch_bounds__(NW * 32, solve_min_blocks<NW>()) k_solve(Batch
             ++G;
             if (gtid == 0) ctl->gr_rounds++;
         }
-        if (gtid == 0 && hlim < INF_H - 1 && (prm.phase != 1 || ctl->gr_front[0] > 0)) ctl->gr_rounds++;
+        if (gtid == 0 && hlim < INF_H - 1 && (prm.phase != 1 || ctl->gr_front > 0)) ctl->gr_rounds++;
         clk.charge(&ctl->t_gr);
         // ------------------------ count active nodes ------------------------
         // warp-uniform loop: the sums of a warp's tiles go out with one

@@ -48,8 +48,6 @@ struct ImgState {
 enum { L_PUSH0 = 0, L_PUSH1, L_PUSH2, L_GR0, L_GR1, L_NLISTS };
 
 // Control block of one solve (zeroed before every launch).
-constexpr int GR_TIMELINE = 32;
-
 struct Ctl {
     unsigned bar_count;
     unsigned bar_gen;
@@ -79,14 +77,14 @@ struct Ctl {
     // timeline of the global relabel of a phase-1 launch (the phase-split
     // diagnostic; %globaltimer ns of block 0): gr_time[0] its start, [1] after
     // round 0, [2] after the first pull check, [3] after the second visits of
-    // the tiles whose check asked for one; gr_front[0] those tiles (the
-    // relabel runs under a height limit, so there is one such round)
-    unsigned long long gr_time[3 + GR_TIMELINE];
-    int gr_front[GR_TIMELINE];
-    // per frontier round of that relabel: the latest end of a tile visit
-    // (%globaltimer ns) and the longest visit (SM cycles); other launches
-    // leave these alone (their global atomics would serialise on one address)
-    unsigned long long gr_front_end[GR_TIMELINE], gr_front_maxcyc[GR_TIMELINE];
+    // the tiles whose check asked for one (the relabel runs under a height
+    // limit, so there is one such round); of that round the tiles, the latest
+    // end of a visit (%globaltimer ns) and the longest visit (SM cycles).  Other
+    // launches leave these alone (their global atomics would serialise on one
+    // address)
+    unsigned long long gr_time[4];
+    int gr_front;
+    unsigned long long gr_front_end, gr_front_maxcyc;
 };
 
 struct Batch {

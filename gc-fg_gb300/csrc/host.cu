@@ -1490,6 +1490,7 @@ gcfg_status gcfg_batch_phase_split(gcfg_batch *b, int n, const int *widths, cons
     SolveParams p = e.prm;
     do {
         if (cudaMemsetAsync(e.d_ctl, 0, sizeof(Ctl), e.st) != cudaSuccess) { rc = GCFG_ERR_CUDA; break; }
+        e.ctl_clean = false;
         p.phase = 1;
         cudaEventRecord(ev[0], e.st);
         if ((rc = launch_solve(e.batch(), p, e.n_tiles, e.st, e.max_grid)) != GCFG_OK) break;
@@ -1504,15 +1505,15 @@ gcfg_status gcfg_batch_phase_split(gcfg_batch *b, int n, const int *widths, cons
         out->push_queue = c1.size[L_PUSH0] + c1.size[L_PUSH1];
         out->relabel_round0_us = (float)((double)(c1.gr_time[1] - c1.gr_time[0]) * 1e-3);
         out->relabel_pull_us = (float)((double)(c1.gr_time[2] - c1.gr_time[1]) * 1e-3);
-        for (int k = 0; k < GR_TIMELINE && k < c1.gr_rounds; ++k) {
-            out->relabel_front_us[k] = (float)((double)(c1.gr_time[3 + k] - c1.gr_time[2 + k]) * 1e-3);
-            out->relabel_front_tiles[k] = c1.gr_front[k];
-            if (c1.gr_front_end[k] > c1.gr_time[2 + k])
-                out->relabel_front_work_us[k] = (float)((double)(c1.gr_front_end[k] - c1.gr_time[2 + k]) * 1e-3);
-            out->relabel_front_maxvisit_kcyc[k] = (float)((double)c1.gr_front_maxcyc[k] * 1e-3);
+        if (c1.gr_rounds > 0) {
+            out->relabel_front_us[0] = (float)((double)(c1.gr_time[3] - c1.gr_time[2]) * 1e-3);
+            out->relabel_front_tiles[0] = c1.gr_front;
+            if (c1.gr_front_end > c1.gr_time[2])
+                out->relabel_front_work_us[0] = (float)((double)(c1.gr_front_end - c1.gr_time[2]) * 1e-3);
+            out->relabel_front_maxvisit_kcyc[0] = (float)((double)c1.gr_front_maxcyc * 1e-3);
         }
         cudaEventElapsedTime(&out->ms_relabel, ev[0], ev[1]);
-        if (c1.total_active == 0) break;  // nothing to push: the solve is over after the relabel
+        if (c1.total_active == 0) break;  // nothing to push within the height limit
         p.phase = 2;  // the control block keeps the first push round's queues
         cudaEventRecord(ev[2], e.st);
         if ((rc = launch_solve(e.batch(), p, e.n_tiles, e.st, e.max_grid)) != GCFG_OK) break;
