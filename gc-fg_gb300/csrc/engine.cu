@@ -875,10 +875,11 @@ struct HandOver {
 // Only rows that changed are written back, the next visit's loads start
 // without a barrier behind the hand-over, and the dependent round trips to
 // memory (the queue's counter, the hand-over's results, the own tile's queue
-// entry) run beside the loads and sweeps.  Device time of a solve, before ->
-// with the adds -> with the write-back -> with the round trips: 1920x1080
-// 212 -> 204 -> 202 -> 200 us, 4096x4096 1069 -> 1012 -> 990 -> 990, 40 uneven
-// images 337 -> 325 -> 321 -> 314, 256 of them 1530 -> 1493 -> 1424 -> 1400.
+// entry) run beside the loads and sweeps.  Device time of a whole call (data
+// term to cuts), before -> with the adds -> with the write-back -> with the
+// round trips: 1920x1080 212 -> 204 -> 202 -> 200 us, 4096x4096 1069 -> 1012 ->
+// 990 -> 990, 40 uneven images 337 -> 325 -> 321 -> 314, 256 of them 1530 -> 1493
+// -> 1424 -> 1400.
 // Fetching the next tile into the L2 cache as well, or dealing the tiles out
 // in turn so that it is known earlier, gave no more (256 images 1385 to 1400
 // us, 4096x4096 997 to 1020): with four blocks per SM a large solve's visits
@@ -1302,9 +1303,11 @@ __global__ void __launch_bounds__(NW * 32, solve_min_blocks<NW>()) k_solve(Batch
     for (int outer = 0; outer < prm.max_outer; ++outer) {
         const int hlim = full || outer >= prm.near_outer ? INF_H - 1 : prm.near_h << (2 * outer);
         // A solve that has come past its first unlimited iteration moves much
-        // flow far: twice the sweeps per visit save it relabels (lambda 1e5,
-        // single 512x512 image, 24 relabels -> 15, 4.26 -> 3.09 ms; 256x256 22 ->
-        // 16, 4.19 -> 3.36; 1024x1024 24 -> 15, 4.94 -> 4.39).
+        // flow far: twice the sweeps per visit save it relabels (lambda 1e5, mean
+        // of ten images: 256x256 13 relabels -> 10, 1.89 -> 1.71 ms, 512x512 18 ->
+        // 12, 2.81 -> 2.33, 1024x768 33 -> 23, 5.66 -> 4.46; 24 sweeps in every
+        // iteration 1.92, 2.62 and 4.75).  Constant penalties of 100 to 600, whose
+        // solves are as long, lose 3% by it on average (-6% to +20%).
         const int max_sweeps = outer > prm.near_outer ? 2 * prm.max_sweeps : prm.max_sweeps;
         if (prm.phase == 2) goto push_rounds;  // the phase-1 launch did the relabel and the count
         if (outer > 0) {

@@ -911,10 +911,11 @@ gcfg_status gcfg_optimize8(gcfg_graph8 *g, int32_t *host_label, gcfg_result *res
     if (want < grid) grid = want > 0 ? want : 1;
     G8 gg = g->g();
     // A height limit for the first iteration pays where edges saturate, as
-    // contrast-sensitive ones do; a constant penalty leaves most of them
-    // open, flow has to travel, and the limited iteration is in the way
-    // (640x480 / 1920x1080, us without -> with: arrays 272 -> 177, 602 -> 393;
-    // penalty 600 963 -> 995, 3344 -> 4285).
+    // contrast-sensitive ones do (640x480 / 1920x1080, us without -> with: arrays
+    // 272 -> 177, 602 -> 393).  A constant penalty leaves most of them open and
+    // flow has to travel: penalty 600 770 -> 862, 2473 -> 2662; penalty 100, where
+    // some saturate, 1803 -> 1719, 2459 -> 2032 (three graphs each; the penalty
+    // given by itself and as arrays).
     P8 prm{g->max_outer, g->rounds < MAX_ROUNDS8 ? g->rounds : MAX_ROUNDS8, g->sweeps, g->varying ? 9 : 0};
     void *args[] = {&gg, &prm};
     GCFG_CK(cudaEventRecord(g->ev0, g->st));
