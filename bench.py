@@ -1,6 +1,8 @@
 """Benchmark: exact min-cut segmentation throughput on GB300.
 
-Prints ONE JSON line (rank 0).  A step = the full hot path over one batch of
+Prints ONE JSON line (rank 0) of at most 2,800 characters (headline()); the
+full record of every leg, some 20,000, goes to standard error as one line that
+begins with "detail: ".  A step = the full hot path over one batch of
 synthetic images: colour-histogram t-links, contrast-sensitive n-links,
 graph build, exact max-flow, both canonical cuts.
 
@@ -99,6 +101,44 @@ B_GR, B_PUSH, B_REACH, B_COUNT, B_BUILD, B_EXTRACT = 4.75, 48, 0.875, 12 / 1024,
 MOVED_GR_VISIT = 768 + 512 + 264 + 4096 + 512 + 128 + 4
 MOVED_GR_TILE = 8 + 128 + 512 + 512 + 264 + 12
 MOVED_PUSH_VISIT = 24576 + 512 + 24576 + 768 + 512 + 8
+
+
+def headline(line):
+    """The printed line: every key of the benchmark's own contract whole, and of
+    the long legs their figures alone.  A line of many thousand characters gets
+    cut on its way through logs, and a cut line holds no number at all."""
+    def pick(d, *keys):
+        return {k: (round(d[k], 4) if isinstance(d[k], float) else d[k]) for k in keys if d.get(k) is not None}
+
+    out = {k: v for k, v in line.items() if not isinstance(v, dict)}
+    out["config"] = {k: v for k, v in line["config"].items() if k not in ("tuning", "cuda_graph")}
+    if line["config"].get("tuning"):
+        out["config"]["tuning"] = pick(line["config"]["tuning"], "push_rounds_per_gr", "max_tile_sweeps",
+                                       "sweeps_per_local_relabel", "blocks_per_sm", "threads_y")
+    for k in ("clocks", "cpu_baseline", "parity"):
+        if k in line:
+            out[k] = line[k]
+    for k in ("e2e", "e2e_sync", "plain_per_image"):
+        if k in line:
+            out[k] = pick(line[k], "value", "unit", "ms_per_step", "h2d_bytes_per_step", "d2h_bytes_per_step",
+                          "flows_equal_batched", "cuts_equal_batched")
+    if "roofline" in line:
+        out["roofline"] = pick(line["roofline"], "bound", "kernel", "achieved", "peak", "unit", "frac", "peak_source",
+                               "traffic", "alg_bytes_per_launch", "avg_launch_us", "share_of_step")
+    if "reference_cuda" in line:
+        out["reference_cuda"] = pick(line["reference_cuda"], "value", "unit", "images", "labels_equal_smax", "unavailable")
+    if "serving" in line:
+        out["serving"] = pick(line["serving"]["served"], "p50_ms", "p99_ms", "mpixel_s_over_busy")
+        out["serving"].update(pick(line["serving"], "p99_target_ms", "p99_met", "results_equal"))
+    if "single_image" in line:
+        out["single_image"] = {k: dict(pick(v, "value", "ms_per_step"), e2e=round(v["e2e"]["value"], 4))
+                               for k, v in line["single_image"].items() if "value" in v}
+    return out
+
+
+def emit(line):
+    print("detail: " + json.dumps(line), file=sys.stderr, flush=True)
+    print(json.dumps(headline(line)), flush=True)
 
 
 def workload(name, rank=0):
@@ -913,7 +953,7 @@ def run_n8(args, rank, world):
             "config": workload_config("n8_640x480", None, world), "clocks": clk}
     line.update({k: v for k, v in leg.items() if k not in ("desc", "value", "unit", "ms_per_step", "steps")})
     if rank == 0:
-        print(json.dumps(line), flush=True)
+        emit(line)
     return 0
 
 
@@ -1247,7 +1287,7 @@ def main():
                                         ref_budget=min(args.ref_cuda_budget, 3.0))
             legs["clocks"] = sclk.stop()
             line["single_image"] = legs
-        print(json.dumps(line), flush=True)
+        emit(line)
     if dist is not None:
         dist.destroy_process_group()
     return 0
