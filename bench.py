@@ -576,7 +576,7 @@ def peak_source(peak_kind):
 
 def phase_record(ms, alg, moved, traffic, peak, **extra):
     """Device time of a phase with three byte counts over it: algorithmic
-    (int32 accounting), moved (what the phase reads and writes in this
+    (B_GR and so on above), moved (what the phase reads and writes in this
     layout) and, when an ncu capture exists, DRAM traffic."""
     r = {"ms": round(ms, 4), "alg_bytes": int(alg), "moved_bytes": int(moved)}
     if ms > 0:
@@ -872,16 +872,16 @@ def n8_leg(torch, gcfg, steps, warmup, peak, peak_kind, ref_budget=5.0):
     o = O.solve8(hdp, hdn, penalty=pen)
     cpu_s = time.perf_counter() - t
     value = W * H / (ms / 1e3) / 1e6
-    # Algorithmic bytes of the solve kernel in the int32 layout (eight
-    # capacity planes): a global relabel reads caps + excess and writes the
-    # height (40 B/px), its count reads excess + height (8 B/px); a tile visit
-    # that had work reads caps + excess + height and writes them (80 B/px), a
-    # visit without work reads excess + height (8 B/px); the cut pass reads
+    # Algorithmic bytes of the solve kernel (eight int32 capacity planes): a
+    # global relabel reads caps + excess for its masks and writes the height
+    # (40 B/px; its count reads the masks); a visit of a 32x8 tile reads caps +
+    # excess + height and writes them (80 B/px, an upper bound: only changes are
+    # added back), a tile that is not due is one stamp (4 B); the cut pass reads
     # excess and writes the mark (8 B/px).
     n = W * H
     tiles8 = ((W + 31) // 32) * ((H + 7) // 8)
     visits, rounds = r["push_tiles"], r["push_rounds"]
-    alg = (r["global_relabels"] * n * (40 + 8) + visits * 256 * 80 + (rounds * tiles8 - visits) * 256 * 8 + n * 8)
+    alg = r["global_relabels"] * n * 40 + visits * 256 * 80 + (rounds * tiles8 - visits) * 4 + n * 8
     avg_solve_ms = sum(solve_ms) / len(solve_ms)
     achieved = alg / (avg_solve_ms / 1e3) / 1e9
     roofline = {"bound": "hbm", "kernel": "k8_solve", "achieved": achieved, "peak": peak, "unit": "GB/s",
@@ -1228,7 +1228,7 @@ def main():
             inside[name] = {"achieved_alg_gbs": round(gbs, 1), "frac_alg": round(gbs / peak, 4), "ms": ms,
                             "alg_bytes": nbytes}
     inside["note"] = ("phase timers inside the whole solve (every global relabel and termination check, every push "
-                      "round), int32-layout bytes")
+                      "round), algorithmic bytes")
     roofline["solve_phases"]["inside_full_solve"] = inside
 
     r0 = recs[0]
